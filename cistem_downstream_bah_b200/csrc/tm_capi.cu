@@ -65,6 +65,7 @@ struct tm_ctx {
     int precision = TM_PRECISION_FP32;
     tmk::GenPlan gen_px{}, gen_py{}, gen_ph{};   // radix plans of X, Y and X/2 (sizes without compiled kernels)
     uint4* dft = nullptr;       // DFT operands of the tensor-core row pass (FP16 form)
+    tmk::CMaps cmaps{};         // C as the compiled geometries' kernels read and write it
     long long rot_capacity = 0;
     bool has_template = false, has_image = false;
     // bookkeeping for decoding the argmax
@@ -264,7 +265,7 @@ struct Impl {
 
     static int run_stages(tm_ctx* c, tmk::BatchArgs& a) {
         LN::prep(a, c->stream);
-        LN::pass_b(a, c->stream, c->nsm);
+        LN::pass_b(a, c->cmaps, c->stream, c->nsm);
         cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return set_err(c, TM_ERR_CUDA, "kernel launch failed: %s", cudaGetErrorString(e));
         return TM_OK;
@@ -284,8 +285,8 @@ struct Impl {
             a.sum = sl.sum;
             a.sumsq = sl.sumsq;
             a.hist = sl.hist;
-            LN::pass_b(a, s, c->nsm);
-            LN::pass_c(a, s);
+            LN::pass_b(a, c->cmaps, s, c->nsm);
+            LN::pass_c(a, c->cmaps, s, c->nsm);
         }
         cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return set_err(c, TM_ERR_CUDA, "kernel launch failed: %s", cudaGetErrorString(e));
@@ -297,9 +298,9 @@ struct Impl {
         if (ev) cudaEventRecord(ev[0], s);
         LN::prep(a, s);
         if (ev) cudaEventRecord(ev[1], s);
-        LN::pass_b(a, s, c->nsm);
+        LN::pass_b(a, c->cmaps, s, c->nsm);
         if (ev) cudaEventRecord(ev[2], s);
-        LN::pass_c(a, s);
+        LN::pass_c(a, c->cmaps, s, c->nsm);
         if (ev) cudaEventRecord(ev[3], s);
         cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return set_err(c, TM_ERR_CUDA, "kernel launch failed: %s", cudaGetErrorString(e));
@@ -896,6 +897,10 @@ int tm_create(const tm_dims* dims, tm_ctx** out) {
     TRY(dalloc(c, &c->norm, B));
     TRY(dalloc(c, &c->A, B * T * XP));
     TRY(dalloc(c, &c->C, B * Y * XP));
+    if (c->var->X > 0) {   // the compiled geometries' kernels go through tensor maps of C
+        cudaError_t e = tmk::c_tensor_maps(&c->cmaps, c->C, (int)XP, (int)Y, (int)B);
+        if (e != cudaSuccess) { *out = c; return set_err(c, TM_ERR_CUDA, "tensor maps: %s", cudaGetErrorString(e)); }
+    }
     TRY(dalloc(c, &c->filter, T * TP));
     TRY(dalloc(c, &c->mip, X * Y));
     TRY(dalloc(c, &c->best, X * Y));
@@ -1446,7 +1451,17 @@ int tm_debug_stage_buffers(tm_ctx* c, const float* projection_filter, const floa
     if (projection) TM_CUDA(c, cudaMemcpy(projection, c->P, sizeof(float) * T * T, cudaMemcpyDeviceToHost));
     if (normalisation) TM_CUDA(c, cudaMemcpy(normalisation, c->norm, sizeof(float2), cudaMemcpyDeviceToHost));
     if (rows) TM_CUDA(c, cudaMemcpy2D(rows, hc * sizeof(float2), c->A, XP * sizeof(float2), hc * sizeof(float2), T, cudaMemcpyDeviceToHost));
-    if (columns) TM_CUDA(c, cudaMemcpy2D(columns, hc * sizeof(float2), c->C, XP * sizeof(float2), hc * sizeof(float2), (size_t)c->Y, cudaMemcpyDeviceToHost));
+    if (columns && c->var->X == 0) {
+        TM_CUDA(c, cudaMemcpy2D(columns, hc * sizeof(float2), c->C, XP * sizeof(float2), hc * sizeof(float2), (size_t)c->Y, cudaMemcpyDeviceToHost));
+    } else if (columns) {
+        // out of the compiled geometries' tiles
+        std::vector<float2> tiles((size_t)c->Y * XP);
+        TM_CUDA(c, cudaMemcpy(tiles.data(), c->C, sizeof(float2) * tiles.size(), cudaMemcpyDeviceToHost));
+        const size_t R = tmk::c_tile_rows(c->Y);
+        for (size_t y = 0; y < (size_t)c->Y; y++)
+            for (size_t k = 0; k < hc; k++)
+                reinterpret_cast<float2*>(columns)[y * hc + k] = tiles[((y / R) * (XP / 4) + k / 4) * 4 * R + (y % R) * 4 + k % 4];
+    }
     return TM_OK;
 }
 

@@ -421,64 +421,139 @@ __device__ __forceinline__ void fft(float2 (&v)[R], int t, float2* buf, const Tw
     });
 }
 
-// The same transform with the twiddle multipliers of every stage supplied by
-// the caller instead of a table lookup and a power tree:
-// src.template issue<s>() starts fetching stage s's multipliers and is called
-// before the stage's barrier, so that the fetch overlaps the barrier and the
-// shared-memory loads; src.template get<s>(u, p) then fills p[1 .. RS-1] with
-// w^1 .. w^(RS-1) of the thread's butterfly u (w as in fft above, DIR applied).
-// Used where the multipliers are per-thread constants held in tensor memory.
-template <int L, int R, int DIR, bool FIRST_SYNC = true, class Src, class Sync>
-__device__ __forceinline__ void fft_pre(float2 (&v)[R], int t, float2* buf, Src& src, Sync sync) {
-    using PL = Plan<L, R>;
-    constexpr int P = PL::P;
-    sfor<PL::stages>([&](auto sc) {
-        constexpr int s = decltype(sc)::value;
-        constexpr int RS = PL::radix(s);
-        constexpr int Ns = PL::ns(s);
-        constexpr bool last = (s == PL::stages - 1);
-        if constexpr (s > 0) {
-            src.template issue<s>();
-            sync();
-            if constexpr (P % 16 == 0 || 16 % P == 0) {
-                const float2* rb = buf + rd_base<P>(t);
-#pragma unroll
-                for (int r = 0; r < R; r++) v[r] = rb[rd_off<P>(r)];
-            } else {
-#pragma unroll
-                for (int r = 0; r < R; r++) v[r] = buf[pad16(t + P * r)];
-            }
-        }
-#pragma unroll
-        for (int u = 0; u < R / RS; u++) {
-            const int b = t + P * u;
-            float2 e[RS];
-#pragma unroll
-            for (int r = 0; r < RS; r++) e[r] = v[u + r * (R / RS)];
-            if constexpr (s > 0) {
-                float2 pw[RS];
-                src.template get<s>(u, pw);
-#pragma unroll
-                for (int r = 1; r < RS; r++) e[r] = cmul(e[r], pw[r]);
-            }
-            dft<RS, DIR>(e);
-            if constexpr (last) {
-#pragma unroll
-                for (int r = 0; r < RS; r++) v[u + r * (R / RS)] = e[r];
-            } else {
-                if (u == 0 && (FIRST_SYNC || s > 0)) sync();
-                if constexpr (RS == R && ((Ns == 1 && 16 % R == 0) || Ns % 16 == 0)) {
-                    float2* wb = buf + wr_base<R>(b, Ns);
-#pragma unroll
-                    for (int r = 0; r < RS; r++) wb[wr_off(r, Ns)] = e[r];
-                } else {
-                    const int idxD = (b / Ns) * Ns * RS + (b % Ns);
-#pragma unroll
-                    for (int r = 0; r < RS; r++) buf[pad16(idxD + r * Ns)] = e[r];
-                }
-            }
-        }
-    });
+// ---- Two transforms at a time -------------------------------------------------------
+// The same element of two independent transforms (two orientations, two columns), real
+// parts and imaginary parts side by side, so that sm_100's two-wide FP32 instructions
+// (add / sub / mul / fma .f32x2) do both with one issue slot; each half is rounded as its
+// scalar form, so a transform gives the same bits in a pair as alone.  The FP32 pipe's
+// lane rate is that of scalar code (122 FADD lanes per clock and SM measured, 126 two-wide):
+// the gain is the issue slots, which bound the transforms of the search (60 % issue active
+// with the FP32 pipe at a third to a half).
+struct Pair {
+    float2 re, im;
+};
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+    float2 r;
+    asm("{\n\t.reg .b64 p, q, s;\n\tmov.b64 p, {%2, %3};\n\tmov.b64 q, {%4, %5};\n\tadd.rn.f32x2 s, p, q;\n\t"
+        "mov.b64 {%0, %1}, s;\n\t}"
+        : "=f"(r.x), "=f"(r.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return r;
+}
+__device__ __forceinline__ float2 sub2(float2 a, float2 b) {
+    float2 r;
+    asm("{\n\t.reg .b64 p, q, s;\n\tmov.b64 p, {%2, %3};\n\tmov.b64 q, {%4, %5};\n\tsub.rn.f32x2 s, p, q;\n\t"
+        "mov.b64 {%0, %1}, s;\n\t}"
+        : "=f"(r.x), "=f"(r.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return r;
+}
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+    float2 r;
+    asm("{\n\t.reg .b64 p, q, s;\n\tmov.b64 p, {%2, %3};\n\tmov.b64 q, {%4, %5};\n\tmul.rn.f32x2 s, p, q;\n\t"
+        "mov.b64 {%0, %1}, s;\n\t}"
+        : "=f"(r.x), "=f"(r.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return r;
+}
+// a b + c
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+    float2 r;
+    asm("{\n\t.reg .b64 p, q, s, t;\n\tmov.b64 p, {%2, %3};\n\tmov.b64 q, {%4, %5};\n\tmov.b64 s, {%6, %7};\n\t"
+        "fma.rn.f32x2 t, p, q, s;\n\tmov.b64 {%0, %1}, t;\n\t}"
+        : "=f"(r.x), "=f"(r.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+    return r;
+}
+__device__ __forceinline__ float2 both(float v) { return make_float2(v, v); }
+__device__ __forceinline__ Pair padd(Pair a, Pair b) { return {add2(a.re, b.re), add2(a.im, b.im)}; }
+__device__ __forceinline__ Pair psub(Pair a, Pair b) { return {sub2(a.re, b.re), sub2(a.im, b.im)}; }
+// a + (DIR i) b and a - (DIR i) b
+template <int DIR>
+__device__ __forceinline__ Pair padd_i(Pair a, Pair b) {
+    if constexpr (DIR < 0) return {add2(a.re, b.im), sub2(a.im, b.re)};
+    else return {sub2(a.re, b.im), add2(a.im, b.re)};
+}
+template <int DIR>
+__device__ __forceinline__ Pair psub_i(Pair a, Pair b) { return padd_i<-DIR>(a, b); }
+// a w for one factor, and a w for a factor of each half (cmul per half: the factor's parts
+// would have to be doubled into register pairs for the two-wide form)
+__device__ __forceinline__ Pair pmul(Pair a, float2 w) {
+    const float2 x = cmul(make_float2(a.re.x, a.im.x), w), y = cmul(make_float2(a.re.y, a.im.y), w);
+    return {make_float2(x.x, y.x), make_float2(x.y, y.y)};
+}
+
+// a conj(b) with the roles of cmul_conj, b per half
+__device__ __forceinline__ Pair pmul_conj(float2 ax, float2 ay, Pair b) {   // a = (ax.x, ay.x), (ax.y, ay.y)
+    const float2 x = cmul_conj(make_float2(ax.x, ay.x), make_float2(b.re.x, b.im.x));
+    const float2 y = cmul_conj(make_float2(ax.y, ay.y), make_float2(b.re.y, b.im.y));
+    return {make_float2(x.x, y.x), make_float2(x.y, y.y)};
+}
+// a (c + i s) for a compile-time factor, two-wide, rounded as cmul
+__device__ __forceinline__ Pair pmulc(Pair a, float c, float s) {
+    return {fma2(a.re, both(c), mul2(a.im, both(-s))), fma2(a.re, both(s), mul2(a.im, both(c)))};
+}
+
+// ROT2: a2 still lacks a factor DIR i
+template <int DIR, bool ROT2 = false>
+__device__ __forceinline__ void pdft4(Pair& a0, Pair& a1, Pair& a2, Pair& a3) {
+    const Pair s02 = ROT2 ? padd_i<DIR>(a0, a2) : padd(a0, a2), d02 = ROT2 ? psub_i<DIR>(a0, a2) : psub(a0, a2);
+    const Pair s13 = padd(a1, a3), d13 = psub(a1, a3);
+    a0 = padd(s02, s13);
+    a2 = psub(s02, s13);
+    a1 = padd_i<DIR>(d02, d13);
+    a3 = psub_i<DIR>(d02, d13);
+}
+
+// dft8 of both halves
+template <int DIR>
+__device__ __forceinline__ void pdft8(Pair* v) {
+    constexpr float h = 0.70710678118654752440f;
+    pdft4<DIR>(v[0], v[2], v[4], v[6]);
+    pdft4<DIR>(v[1], v[3], v[5], v[7]);
+    // v[3] W8 = h (v + DIR i v), v[7] W8^3 = -h (v - DIR i v): the factor h inside the last additions
+    const Pair t3 = padd_i<DIR>(v[3], v[3]), t7 = psub_i<DIR>(v[7], v[7]);
+    const Pair a0 = v[0], a1 = v[2], a2 = v[4], a3 = v[6], b0 = v[1], b2 = v[5];
+    v[0] = padd(a0, b0);
+    v[4] = psub(a0, b0);
+    v[1] = {fma2(t3.re, both(h), a1.re), fma2(t3.im, both(h), a1.im)};
+    v[5] = {fma2(t3.re, both(-h), a1.re), fma2(t3.im, both(-h), a1.im)};
+    v[2] = padd_i<DIR>(a2, b2);
+    v[6] = psub_i<DIR>(a2, b2);
+    v[3] = {fma2(t7.re, both(-h), a3.re), fma2(t7.im, both(-h), a3.im)};
+    v[7] = {fma2(t7.re, both(h), a3.re), fma2(t7.im, both(h), a3.im)};
+}
+
+// The 16-point DFT of both halves (rounded as dft16) as its two levels of four 4-point
+// transforms with the constants between, so that a caller can put loads, factors and stores
+// between the groups of four: level 1 takes x[r2], x[4 + r2], x[8 + r2], x[12 + r2], level 2 leaves
+// X[q1], X[q1 + 4], X[q1 + 8], X[q1 + 12].  pdft16_mid takes element (q1, r2) of level 1's results
+// at v[4 q1 + r2] or at v[4 r2 + q1] (its factors are symmetric); the factor DIR i of (2, 2),
+// v[10], is left to level 2 of q1 = 2 (pdft4's ROT2).
+template <int DIR>
+__device__ __forceinline__ void pdft16_mid(Pair* v) {
+    constexpr float c1 = 0.92387953251128675613f, s1 = 0.38268343236508977173f, h = 0.70710678118654752440f;
+    constexpr float sg = DIR < 0 ? -1.f : 1.f;
+    v[5] = pmulc(v[5], c1, sg * s1);
+    v[6] = pmulc(v[6], h, sg * h);
+    v[7] = pmulc(v[7], s1, sg * c1);
+    v[9] = pmulc(v[9], h, sg * h);
+    v[11] = pmulc(v[11], -h, sg * h);
+    v[13] = pmulc(v[13], s1, sg * c1);
+    v[14] = pmulc(v[14], -h, sg * h);
+    v[15] = pmulc(v[15], -c1, -sg * s1);
+}
+
+template <int RS, int DIR>
+__device__ __forceinline__ void pdft(Pair* v) {
+    if constexpr (RS == 8) pdft8<DIR>(v);
+    else if constexpr (RS == 4) pdft4<DIR>(v[0], v[1], v[2], v[3]);
+    else {
+        static_assert(RS == 2, "unsupported radix");
+        const Pair a = v[0], b = v[1];
+        v[0] = padd(a, b);
+        v[1] = psub(a, b);
+    }
 }
 
 }  // namespace tmfft

@@ -28,6 +28,7 @@
 // (ClipIntoLargerRealSpace2D, image.cpp:8398-8465), the forward-FFT scaling
 // 1/N and the zeroed central pixel are folded into I' once per micrograph.
 #pragma once
+#include <cuda.h>
 #include <cuda_fp16.h>
 #include <float.h>
 #include "tm_fft.cuh"
@@ -56,6 +57,29 @@ __host__ __device__ constexpr int prune_len(int T, int N, int V) {
 // heights with a factor 3
 __host__ __device__ constexpr int col_radix(int Y) { return Y % 3 == 0 ? 18 : 16; }
 
+// Layout of the FP32 correlation spectra C between passes B and C of a height Y: tiles of
+// c_tile_rows(Y) rows x 4 columns, C[o][y / R][kx / 4][y % R][kx % 4].  A column pass writes 4
+// columns of every row of one orientation: in this layout whole tiles of 256 bytes (128
+// where 8 does not divide the height) instead of 32-byte pieces of rows 16 KB apart, which the
+// memory takes at 5.5 instead of 2.7-3.0 TB/s (a store-only kernel, 2.15 GB, 4096 x 4096).  The
+// row pass gathers a row's 32-byte pieces by tensor-map copies; the blocks on the R rows
+// of a tile read it at about the same time, through the L2 (4.8-5.5 TB/s in a load-only
+// kernel, against 7.2 for whole rows; it needs 2.8).
+__host__ __device__ constexpr int c_tile_rows(int Y) { return Y % 8 == 0 ? 8 : 4; }
+template <int Y>
+__host__ __device__ constexpr size_t c_index(int o, int y, int kx, int XP) {
+    constexpr int R = c_tile_rows(Y);
+    static_assert(Y % R == 0, "heights are whole tiles");
+    return (((size_t)o * (Y / R) + y / R) * (XP / 4) + kx / 4) * (4 * R) + (y % R) * 4 + kx % 4;
+}
+// A row of C in the row pass's shared memory: its XP / 4 column groups arrive in c_row_boxes(XP)
+// copies of c_row_box(XP) groups (at most 256, a multiple of 4 for 128-byte aligned pieces)
+__host__ __device__ constexpr int c_row_boxes(int XP) { return (XP / 4 + 255) / 256; }
+__host__ __device__ constexpr int c_row_box(int XP) {
+    return ((XP / 4 + c_row_boxes(XP) - 1) / c_row_boxes(XP) + 3) / 4 * 4;
+}
+__host__ __device__ constexpr int c_row_len(int XP) { return 4 * c_row_boxes(XP) * c_row_box(XP); }   // float2
+
 struct BatchArgs {
     int nb;                       // orientations in this batch
     int orient0;                  // index of the batch's first orientation within the plane
@@ -68,7 +92,7 @@ struct BatchArgs {
     double* rowstat;              // nb * T * 4
     float2* norm;                 // nb: (edge mean, 1/sigma)
     float2* A;                    // nb * T * XP
-    float2* C;                    // nb * Y * XP
+    float2* C;                    // nb * Y * XP, tiled (c_index); the FP16 form's own layout
     const float2* Ip;             // Y * XP prepared micrograph spectrum
     float* mip;                   // Y * X
     int* best;                    // Y * X
@@ -503,7 +527,7 @@ __device__ __forceinline__ void tmem_put_values(uint32_t taddr, const float* f) 
     }
 }
 
-// RB = 0: C[o][y][kx] in FP32 complex.  RB > 0 (the FP16 form): C in FP16
+// RB = 0: FP32 complex, tiled (c_index).  RB > 0 (the FP16 form): C in FP16
 // complex times 2^half_scale_exp, rows interleaved in blocks of RB,
 // C16[o][y / RB][kx][y % RB], so that a warp's stores (8 consecutive rows of 4
 // columns) fill whole 32-byte sectors and the tensor-core row pass reads a
@@ -675,9 +699,8 @@ k_pass_b(BatchArgs a, int ngroups) {
                     __stcs(reinterpret_cast<unsigned int*>(Co + (size_t)r * P * XP), *reinterpret_cast<const unsigned int*>(&hv));
                 }
             } else if constexpr (G == 1) {
-                float2* Co = a.C + (size_t)o * Y * XP + kx0 + col;
 #pragma unroll
-                for (int r = 0; r < V; r++) __stcs(Co + (size_t)(j + P * r) * XP, v[r]);   // streaming
+                for (int r = 0; r < V; r++) __stcs(a.C + c_index<Y>(o, j + P * r, kx0 + col, XP), v[r]);   // streaming
             } else {
                 sync();   // every thread has read its last-stage inputs from colbuf
 #pragma unroll
@@ -685,12 +708,12 @@ k_pass_b(BatchArgs a, int ngroups) {
             }
         }
         if constexpr (G > 1) {
-            // the item's WG columns, row by row: whole 32-byte sectors per row
+            // the item's 4 columns: whole tiles
+            static_assert(WG == 4, "chunks written together are one tile wide");
             sync();
-            float2* Co = a.C + (size_t)o * Y * XP + kx0;
             for (int e = tid; e < Y * WG; e += NT) {
                 const int row = e / WG, cc = e % WG;
-                __stcs(Co + (size_t)row * XP + cc, exch[cc * PB::CS + tmfft::pad16(row)]);   // streaming
+                __stcs(a.C + c_index<Y>(o, row, kx0 + cc, XP), exch[cc * PB::CS + tmfft::pad16(row)]);   // streaming
             }
         }
     }
@@ -718,42 +741,46 @@ k_pass_b(BatchArgs a, int ngroups) {
 // DFT.  Per item (4 columns of one orientation) that is two block barriers
 // instead of the six of k_pass_b's Stockham stages.
 //
-// Roles: residue phases -- warp w holds residue s = w >> 1 of columns
-// 2 (w & 1) + (lane >> 4), lane q = lane & 15; final phase -- thread t holds
-// row m' = t >> 2 of column t & 3 (a warp stores 8 rows x 4 columns, whole
-// 32-byte row sectors).  The block buffer is blk[c][m'][s] (row stride 17,
-// column stride CS = 4 mod 16: conflict-free 8-byte accesses in every phase).
-// A warp's transposes use the block-buffer ranges that the same warp reads in
-// the final phase, so they need no barrier of their own: nobody else touches
-// those ranges between the warp's final read and the next block-wide write.
+// Two adjacent columns go through a thread side by side (tmfft::Pair): additions and the
+// constants of the 16-point transforms take one instruction for both, the twiddles are
+// fetched once, and shared memory is accessed 16 bytes at a time.
+//
+// Roles: residue phases -- warp s holds residue s, lane 2 q + cp the columns 2 cp and 2 cp + 1
+// of line q; final phase -- thread 2 m' + cp holds row m' of those columns.  The block buffer is
+// blk[s][m'][cp], 16 bytes each: every phase accesses 128 adjacent bytes per 8 lanes.  In the
+// final phase a thread puts its 16 output rows m' + 256 M back where it read its 16 residues, so
+// that the buffer becomes the item's 512 tiles of C, [M][m'][cp], and two tensor-map stores
+// write it to memory while the next item's residue phases run (with stores from the
+// threads, all of which reach them together, the pass took 3.85 ms per 128 orientations against 2.93 with
+// the stores left out).  A warp's transposes have buffers of their own, of 8 bytes per element
+// for want of shared memory: the real parts of the column pairs go first, then the imaginary parts.
 struct PassBRg {
-    static constexpr int T = 256, Y = 4096, W = 4, NT = 1024;
-    static constexpr int RS = 17;                       // row stride of blk (float2)
-    static constexpr int CS = 256 * RS + 4;             // column stride, == 4 (mod 16)
-    static constexpr int APITCH = 260;                  // A staging: [c][row], 4 columns
-    static constexpr size_t EXCH = sizeof(float2) * W * CS;
-    static constexpr size_t ASZ = sizeof(float2) * W * APITCH;
-    static constexpr int ABUFS = 3;                     // rows of A prefetched two items ahead
-    static constexpr size_t TWB = sizeof(float2) * NT;   // per-thread twiddle W256^(-q)
+    static constexpr int T = 256, Y = 4096, W = 4, NT = 512;
+    static constexpr int RS = 17;                       // row stride of a transpose buffer (float2)
+    static constexpr int SCR = 16 * RS + 8;             // one column pair's, == 8 (mod 16)
+    static constexpr size_t EXCH = sizeof(float4) * 16 * 256 * 2;
+    static constexpr size_t SCRS = sizeof(float2) * 16 * 2 * SCR;
+    static constexpr size_t ASZ = sizeof(float4) * 2 * T;   // A staging: [row][column pair]
+    static constexpr int ABUFS = 2;                     // rows of A prefetched one item ahead
     static constexpr int MAX_ITEMS = 2048;              // a block's item list (group << 16 | orientation)
     static constexpr size_t LIST = sizeof(int) * MAX_ITEMS;
-    static constexpr size_t SMEM = EXCH + ABUFS * ASZ + TWB + LIST + 64;
-    // 8 warps per lane quadrant x 32 columns of I' (columns 0-255), and x 32 columns of
-    // the thread's twiddles W4096^(-(q + 16 r) s) (columns 256-511)
+    static constexpr size_t SMEM = EXCH + SCRS + ABUFS * ASZ + LIST + 64;
+    // 4 warps per lane quadrant x 64 columns of I' (columns 0-255), 32 of the twiddles
+    // W4096^(-(q + 16 r) s) (256-383) and 32 of the powers W256^(-q r) (384-511)
     static constexpr uint32_t TMEM_COLS = 512;
     static_assert(SMEM <= 232448, "pass B block exceeds shared memory");
 };
 
 __global__ void __launch_bounds__(PassBRg::NT, 1)
-k_pass_b_rg(BatchArgs a, int ngroups) {
+k_pass_b_rg(BatchArgs a, const __grid_constant__ CUtensorMap cmap, int ngroups) {
     using PB = PassBRg;
-    constexpr int T = PB::T, Y = PB::Y, RS = PB::RS, CS = PB::CS, AP = PB::APITCH;
-    extern __shared__ __align__(16) unsigned char smem_b[];
-    float2* const blk = reinterpret_cast<float2*>(smem_b);
-    float2* const abuf = reinterpret_cast<float2*>(smem_b + PB::EXCH);
-    float2* const twt = reinterpret_cast<float2*>(smem_b + PB::EXCH + PB::ABUFS * PB::ASZ);
-    int* const items = reinterpret_cast<int*>(smem_b + PB::EXCH + PB::ABUFS * PB::ASZ + PB::TWB);
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem_b + PB::EXCH + PB::ABUFS * PB::ASZ + PB::TWB + PB::LIST);
+    using tmfft::Pair;
+    constexpr int T = PB::T, Y = PB::Y, RS = PB::RS;
+    extern __shared__ __align__(128) unsigned char smem_b[];
+    float4* const blk = reinterpret_cast<float4*>(smem_b);
+    float4* const abuf = reinterpret_cast<float4*>(smem_b + PB::EXCH + PB::SCRS);
+    int* const items = reinterpret_cast<int*>(smem_b + PB::EXCH + PB::SCRS + PB::ABUFS * PB::ASZ);
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem_b + PB::EXCH + PB::SCRS + PB::ABUFS * PB::ASZ + PB::LIST);
     const int tid = threadIdx.x;
     // this block's items (the launcher checks that they fit the list)
     int n_items;
@@ -771,162 +798,247 @@ k_pass_b_rg(BatchArgs a, int ngroups) {
         tmptx::tmem_alloc(tmem_slot, PB::TMEM_COLS);
         tmptx::tmem_relinquish();
     }
-    // the item's 256 rows of A, column-major into the staging buffer [c][row]
-    // (thread: row tid / 4, column tid % 4); items are (column group, orientation),
-    // orientation fastest
-    const float2* const Asrc = a.A + (size_t)(tid >> 2) * a.XP + (tid & 3);
-    const uint32_t adst = tmptx::smem_u32(abuf + (tid & 3) * AP + (tid >> 2));
+    // the item's 256 rows of A into the staging buffer (thread: row tid / 2, column pair
+    // tid % 2); items are (column group, orientation), orientation fastest
+    const float2* const Asrc = a.A + (size_t)(tid >> 1) * a.XP + 2 * (tid & 1);
+    const uint32_t adst = tmptx::smem_u32(abuf + tid);
     auto issue_rows = [&](int grp, int oo, int buf) {
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(adst + buf * (uint32_t)(PB::ASZ)),
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(adst + buf * (uint32_t)(PB::ASZ)),
                      "l"(Asrc + (size_t)oo * T * a.XP + grp * 4)
                      : "memory");
     };
-    // this thread's W256^(-q) in shared memory, indexed by thread (conflict-free reads)
-    twt[tid] = a.twy.template w<-1>(16 * (tid & 15), Y);
-    __syncthreads();   // the item list
+    tmptx::tmem_fence_before_sync();
+    __syncthreads();   // the item list, the TMEM address
+    tmptx::tmem_fence_after_sync();
     issue_rows(items[0] >> 16, items[0] & 0xffff, 0);
     tmptx::cp_async_commit();
-    if (n_items > 1) issue_rows(items[1] >> 16, items[1] & 0xffff, 1);
-    tmptx::cp_async_commit();
-    tmptx::cp_async_wait<1>();
-    tmptx::tmem_fence_before_sync();
-    __syncthreads();
-    tmptx::tmem_fence_after_sync();
-    const uint32_t tmem = *tmem_slot + ((uint32_t)(32 * ((tid >> 5) & 3)) << 16) + (uint32_t)(32 * (tid >> 7));
-    const uint32_t tmw = tmem + 256;   // the twiddles W4096^(-(q + 16 r) s) of the residue phases
+    const int s = tid >> 5, q = (tid >> 1) & 15, cp = tid & 1;   // residue, line, column pair
+    const uint32_t tmem = *tmem_slot + ((uint32_t)(32 * (s & 3)) << 16);
+    const uint32_t tmi = tmem + 64 * (s >> 2);         // this thread's I' values
+    const uint32_t tmw = tmem + 256 + 32 * (s >> 2);   // W4096^(-(q + 16 r) s), r = 0..15
+    const uint32_t tmq = tmem + 384 + 32 * (s >> 2);   // W256^(-q r) by the product tree, r = 0..15
     {
-        const int s = tid >> 6, q = tid & 15;
-#pragma unroll 1
-        for (int h = 0; h < 2; h++) {
-            float wb[16];
+        float2 one[16];
 #pragma unroll
-            for (int r = 0; r < 8; r++) {
-                const float2 w = a.twy.template w<-1>((q + 16 * (8 * h + r)) * s, Y);
-                wb[2 * r] = w.x;
-                wb[2 * r + 1] = w.y;
+        for (int r = 0; r < 16; r++) one[r] = make_float2(1.f, 0.f);
+        tmfft::apply_twiddles<16>(one, a.twy.template w<-1>(16 * q, Y));   // 1 w^r = w^r
+        float wb[16];
+        // in the order of the transforms' groups of four: r = g, g + 4, g + 8, g + 12 for g = 0..3
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+                const int r = 2 * h + i / 4 + 4 * (i % 4);
+                const float2 w = a.twy.template w<-1>((q + 16 * r) * s, Y);
+                wb[2 * i] = w.x;
+                wb[2 * i + 1] = w.y;
             }
             tmptx::tmem_st16(tmw + 16 * h, wb);
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+                const int r = 2 * h + i / 4 + 4 * (i % 4);
+                wb[2 * i] = one[r].x;
+                wb[2 * i + 1] = one[r].y;
+            }
+            tmptx::tmem_st16(tmq + 16 * h, wb);
         }
         tmptx::tmem_wait_st();
     }
+    tmptx::cp_async_wait<0>();
+    __syncthreads();   // the first item's rows
     int cur_group = -1;
-    int buf = 0;
+    auto put = [](float4* at, Pair p) { *at = make_float4(p.re.x, p.re.y, p.im.x, p.im.y); };
+    auto get = [](const float4* at) {
+        const float4 f = *at;
+        return Pair{make_float2(f.x, f.y), make_float2(f.z, f.w)};
+    };
 #pragma unroll 1
     for (int it = 0; it < n_items; it++) {
         const int group = items[it] >> 16, o = items[it] & 0xffff;
-        // residue phases: residue s = warp / 2, column c = 2 (warp % 2) + lane / 16, lane q = lane % 16
-        const int s = tid >> 6, q = tid & 15, c = (tid >> 4) & 3;
         {
-            // rows of item it + 2 into the buffer that item it - 1 used
-            if (it + 2 < n_items) issue_rows(items[it + 2] >> 16, items[it + 2] & 0xffff, buf == 0 ? 2 : buf - 1);
+            // rows of item it + 1 into the buffer that item it - 1 used
+            if (it + 1 < n_items) issue_rows(items[it + 1] >> 16, items[it + 1] & 0xffff, (it + 1) & 1);
             tmptx::cp_async_commit();
         }
         if (group != cur_group) {
-            // this thread's 16 I' values, k = s + 16 q + 256 r, into its TMEM columns
-            const float2* Ig = a.Ip + (size_t)(s + 16 * q) * a.XP + group * 4 + c;
+            // this thread's 16 I' values of two columns, k = s + 16 q + 256 r, as column pairs of
+            // the real and the imaginary parts
+            const float4* Ig = reinterpret_cast<const float4*>(a.Ip + (size_t)(s + 16 * q) * a.XP + group * 4 + 2 * cp);
 #pragma unroll 1
-            for (int h = 0; h < 2; h++) {
+            for (int h = 0; h < 4; h++) {
                 float ib[16];
 #pragma unroll
-                for (int r = 0; r < 8; r++) {
-                    const float2 iv = __ldg(Ig + (size_t)(256 * (8 * h + r)) * a.XP);
-                    ib[2 * r] = iv.x;
-                    ib[2 * r + 1] = iv.y;
+                for (int r = 0; r < 4; r++) {
+                    const float4 iv = __ldg(Ig + (size_t)(128 * (h + 4 * r)) * a.XP);
+                    ib[4 * r] = iv.x;
+                    ib[4 * r + 1] = iv.z;
+                    ib[4 * r + 2] = iv.y;
+                    ib[4 * r + 3] = iv.w;
                 }
-                tmptx::tmem_st16(tmem + 16 * h, ib);
+                tmptx::tmem_st16(tmi + 16 * h, ib);
             }
             tmptx::tmem_wait_st();
             cur_group = group;
         }
-        // transposes: row rho (0..15) of this half-warp's 16 x 16 block sits in the
-        // final-phase ranges of this warp (columns c % 2 and c % 2 + 2, 8 rows of m' each)
-        float2* const scr = blk + (c & 1) * CS + 136 * (tid >> 5);
-#define TM_RG_ROW(rho) (scr + ((rho) >> 3) * (2 * CS) + ((rho) & 7) * RS)
-        float2 v[16];
-        // forward: b[n] = a[n] W4096^(-n s) for n = q + 16 r, 16-point DFT over r (-> k1)
+        // this column pair's transpose buffer: 16 x 16 real or imaginary parts
+        float2* const scr = reinterpret_cast<float2*>(smem_b + PB::EXCH) + (2 * s + cp) * PB::SCR;
+        // Each 16-point transform goes by groups of four, with the group's loads before its first
+        // level and its factors and stores after its second, so that the FP32 pipe and shared
+        // memory are busy at the same time (in phases over all 16 values they took turns, all
+        // warps being in the same phase: 4.09 ms per 128 orientations).  The factors come from
+        // TMEM a group ahead, into the halves of wb in turn.
+        Pair v[16];
+        float wb[16];
+        auto first = [&](uint32_t col) {
+            tmptx::tmem_ld8(col, wb);
+            tmptx::tmem_ld8(col + 8, wb + 8);
+        };
+        auto arrived = [&] { tmptx::tmem_wait_ld8x2(wb, wb + 8); };
+        auto next = [&](uint32_t col, int g) {
+            if (g < 2) tmptx::tmem_ld8(col + 16 + 8 * g, wb + 8 * (g & 1));
+        };
+        auto factor = [&](int g, int k) { return make_float2(wb[8 * (g & 1) + 2 * k], wb[8 * (g & 1) + 2 * k + 1]); };
+        auto mul_by_conj = [](Pair z, float2 w) {
+            const float2 x = cmul_conj(make_float2(z.re.x, z.im.x), w), y = cmul_conj(make_float2(z.re.y, z.im.y), w);
+            return Pair{make_float2(x.x, y.x), make_float2(x.y, y.y)};
+        };
+        // forward: b[n] = a[n] W4096^(-n s) for n = q + 16 r, 16-point DFT over r (-> k1), W256^(-q k1)
         {
-            const float2* ac = abuf + buf * (PB::W * AP) + c * AP + q;
-            float wb[16];
+            const float4* ac = abuf + (it & 1) * (2 * T) + (tid & 31);
+            first(tmw);
+            tmfft::sfor<4>([&](auto gc) {
+                constexpr int g = decltype(gc)::value;
+                arrived();
 #pragma unroll
-            for (int h = 0; h < 2; h++) {
-                tmptx::tmem_ld16(tmw + 16 * h, wb);
-                tmptx::tmem_wait_ld16(wb);
+                for (int k = 0; k < 4; k++) {
+                    const float4 f = ac[32 * (g + 4 * k)];
+                    v[g + 4 * k] = tmfft::pmul({make_float2(f.x, f.z), make_float2(f.y, f.w)}, factor(g, k));
+                }
+                next(tmw, g);
+                tmfft::pdft4<-1>(v[g], v[4 + g], v[8 + g], v[12 + g]);
+            });
+        }
+        first(tmq);
+        tmfft::pdft16_mid<-1>(v);
+        tmfft::sfor<4>([&](auto gc) {
+            constexpr int g = decltype(gc)::value;
+            tmfft::pdft4<-1, g == 2>(v[4 * g], v[4 * g + 1], v[4 * g + 2], v[4 * g + 3]);
+            arrived();
 #pragma unroll
-                for (int r = 0; r < 8; r++) v[8 * h + r] = cmul(ac[16 * (8 * h + r)], make_float2(wb[2 * r], wb[2 * r + 1]));
+            for (int k = 0; k < 4; k++) {   // row n1 = q, column k1 = g + 4 k
+                if (g + k > 0) v[4 * g + k] = tmfft::pmul(v[4 * g + k], factor(g, k));
+                scr[RS * q + g + 4 * k] = v[4 * g + k].re;
             }
-        }
-        tmfft::dft16<-1>(v);
-        tmfft::apply_twiddles<16>(v, twt[tid]);                         // W256^(-q k1)
-        __syncwarp();   // the warp's final-phase reads of the previous item are done
-#pragma unroll
-        for (int r = 0; r < 16; r++) TM_RG_ROW(q)[r] = v[r];           // row n1 = q, column k1 = r
-        __syncwarp();
-#pragma unroll
-        for (int r = 0; r < 16; r++) v[r] = TM_RG_ROW(r)[q];           // thread k1 = q holds n1 = r
-        __syncwarp();
-        tmfft::dft16<-1>(v);                                           // -> k2: F[s + 16 q + 256 r]
-        // Z = I' conj(F)
+            next(tmq, g);
+        });
         {
-            float iv[16];
-            tmptx::tmem_ld16(tmem, iv);
-            tmptx::tmem_wait_ld16(iv);
+            float2 im[16];   // X[r] of the transform just done
 #pragma unroll
-            for (int r = 0; r < 8; r++) v[r] = cmul_conj(make_float2(iv[2 * r], iv[2 * r + 1]), v[r]);
-            tmptx::tmem_ld16(tmem + 16, iv);
-            tmptx::tmem_wait_ld16(iv);
+            for (int r = 0; r < 16; r++) im[r] = v[4 * (r % 4) + r / 4].im;
+            __syncwarp();
 #pragma unroll
-            for (int r = 0; r < 8; r++) v[8 + r] = cmul_conj(make_float2(iv[2 * r], iv[2 * r + 1]), v[8 + r]);
+            for (int r = 0; r < 16; r++) v[r].re = scr[RS * r + q];   // lane k1 = q holds n1 = r
+            __syncwarp();
+#pragma unroll
+            for (int r = 0; r < 16; r++) scr[RS * q + r] = im[r];
         }
-        // inverse, residue part: 16-point DFT over k2 (-> m1), W256^(m1 q), transpose,
+        __syncwarp();
+#pragma unroll
+        for (int g = 0; g < 4; g++) {
+#pragma unroll
+            for (int k = 0; k < 4; k++) v[g + 4 * k].im = scr[RS * (g + 4 * k) + q];
+            tmfft::pdft4<-1>(v[g], v[4 + g], v[8 + g], v[12 + g]);
+        }
+        __syncwarp();
+        first(tmi);
+        tmfft::pdft16_mid<-1>(v);
+        // -> k2: F[s + 16 q + 256 r]; Z = I' conj(F); inverse: level 1 of the 16-point DFT over k2 (-> m1)
+        tmfft::sfor<4>([&](auto gc) {
+            constexpr int g = decltype(gc)::value;
+            tmfft::pdft4<-1, g == 2>(v[4 * g], v[4 * g + 1], v[4 * g + 2], v[4 * g + 3]);
+            arrived();
+#pragma unroll
+            for (int k = 0; k < 4; k++)
+                v[4 * g + k] = tmfft::pmul_conj(make_float2(wb[4 * k], wb[4 * k + 1]), make_float2(wb[4 * k + 2], wb[4 * k + 3]), v[4 * g + k]);
+            if constexpr (g < 3) first(tmi + 16 * (g + 1));
+            else first(tmq);
+            tmfft::pdft4<+1>(v[4 * g], v[4 * g + 1], v[4 * g + 2], v[4 * g + 3]);
+        });
+        tmfft::pdft16_mid<+1>(v);
+        // W256^(m1 q), transpose
+        tmfft::sfor<4>([&](auto gc) {
+            constexpr int g = decltype(gc)::value;
+            tmfft::pdft4<+1, g == 2>(v[g], v[4 + g], v[8 + g], v[12 + g]);
+            arrived();
+#pragma unroll
+            for (int k = 0; k < 4; k++) {   // row k1 = q, column m1 = g + 4 k
+                if (g + k > 0) v[g + 4 * k] = tmfft::pmul(v[g + 4 * k], tmfft::conjf2(factor(g, k)));
+                scr[RS * q + g + 4 * k] = v[g + 4 * k].re;
+            }
+            next(tmq, g);
+        });
+        __syncwarp();
+#pragma unroll
+        for (int r = 0; r < 16; r++) v[r].re = scr[RS * r + q];   // lane m1 = q holds k1 = r
+        __syncwarp();
+#pragma unroll
+        for (int r = 0; r < 16; r++) scr[RS * q + r] = v[r].im;
+        __syncwarp();
         // 16-point DFT over k1 (-> m2), then W4096^(s (m1 + 16 m2))
-        tmfft::dft16<+1>(v);
-        tmfft::apply_twiddles<16>(v, tmfft::conjf2(twt[tid]));
 #pragma unroll
-        for (int r = 0; r < 16; r++) TM_RG_ROW(q)[r] = v[r];           // row k1 = q, column m1 = r
-        __syncwarp();
+        for (int g = 0; g < 4; g++) {
 #pragma unroll
-        for (int r = 0; r < 16; r++) v[r] = TM_RG_ROW(r)[q];           // thread m1 = q holds k1 = r
-#undef TM_RG_ROW
-        tmfft::dft16<+1>(v);                                           // -> m2
-        {
-            float wb[16];
-#pragma unroll
-            for (int h = 0; h < 2; h++) {
-                tmptx::tmem_ld16(tmw + 16 * h, wb);
-                tmptx::tmem_wait_ld16(wb);
-#pragma unroll
-                for (int r = 0; r < 8; r++) v[8 * h + r] = cmul_conj(v[8 * h + r], make_float2(wb[2 * r], wb[2 * r + 1]));
-            }
+            for (int k = 0; k < 4; k++) v[g + 4 * k].im = scr[RS * (g + 4 * k) + q];
+            tmfft::pdft4<+1>(v[g], v[4 + g], v[8 + g], v[12 + g]);
         }
-        // every warp is done with its transposes (which overlap other warps' final ranges)
+        first(tmw);
+        tmfft::pdft16_mid<+1>(v);
+        tmfft::sfor<4>([&](auto gc) {
+            constexpr int g = decltype(gc)::value;
+            tmfft::pdft4<+1, g == 2>(v[4 * g], v[4 * g + 1], v[4 * g + 2], v[4 * g + 3]);
+            arrived();
+#pragma unroll
+            for (int k = 0; k < 4; k++) v[4 * g + k] = mul_by_conj(v[4 * g + k], factor(g, k));
+            next(tmw, g);
+        });
+        // the previous item's stores have read the block buffer
+        if (tid == 0) tmptx::bulk_wait_read();
         __syncthreads();
-        {
-            float2* bw = blk + c * CS + q * RS + s;
 #pragma unroll
-            for (int r = 0; r < 16; r++) bw[16 * RS * r] = v[r];         // G_s[m' = q + 16 r]
-        }
-        tmptx::cp_async_wait<1>();   // the next item's rows (issued at the top of the previous item)
+        for (int i = 0; i < 16; i++) put(blk + (s * 256 + q + 16 * (i / 4 + 4 * (i % 4))) * 2 + cp, v[i]);   // G_s[m' = q + 16 r]
+        tmptx::cp_async_wait<0>();   // the next item's rows (issued at the top of this item)
         __syncthreads();
-        // final phase: thread holds row m' = tid / 4 of column tid % 4
-        {
-            const float2* br = blk + (tid & 3) * CS + (tid >> 2) * RS;
+        // final phase: row m' = tid / 2 of column pair tid % 2; 16-point DFT over the residues (-> M)
 #pragma unroll
-            for (int r = 0; r < 16; r++) v[r] = br[r];                  // residues s = r of row m'
+        for (int g = 0; g < 4; g++) {
+#pragma unroll
+            for (int k = 0; k < 4; k++) v[g + 4 * k] = get(blk + 512 * (g + 4 * k) + tid);
+            tmfft::pdft4<+1>(v[g], v[4 + g], v[8 + g], v[12 + g]);
         }
-        tmfft::dft16<+1>(v);                                           // -> M
-        {
-            // streaming stores (evict first): pass C reads the intermediate only after the
-            // whole launch, far more than L2 holds (4.17 -> 4.02 ms per 128 orientations)
-            float2* Co = a.C + ((size_t)o * Y + (tid >> 2)) * a.XP + group * 4 + (tid & 3);
-            const size_t rstep = (size_t)256 * a.XP;
+        tmfft::pdft16_mid<+1>(v);
+        tmfft::sfor<4>([&](auto gc) {
+            constexpr int g = decltype(gc)::value;
+            tmfft::pdft4<+1, g == 2>(v[4 * g], v[4 * g + 1], v[4 * g + 2], v[4 * g + 3]);
 #pragma unroll
-            for (int r = 0; r < 16; r++) {
-                __stcs(Co, v[r]);
-                Co += rstep;
+            for (int k = 0; k < 4; k++) {
+                const Pair z = v[4 * g + k];
+                blk[512 * (g + 4 * k) + tid] = make_float4(z.re.x, z.im.x, z.re.y, z.im.y);
             }
+        });
+        // the item's tiles are complete once every warp has come here; only warp 0 waits for that
+        tmptx::fence_proxy_async_smem();
+        if (s == 0) {
+            asm volatile("bar.sync 1, 512;" ::: "memory");
+            if (tid == 0) {
+                tmptx::tensor3_s2g(&cmap, 0, group, o * (Y / 8), blk);
+                tmptx::tensor3_s2g(&cmap, 0, group, o * (Y / 8) + 256, blk + 4096);
+                tmptx::bulk_commit();
+            }
+        } else {
+            asm volatile("bar.arrive 1, 512;" ::: "memory");
         }
-        buf = buf == 2 ? 0 : buf + 1;
     }
+    if (tid == 0) tmptx::bulk_wait_all();
     tmptx::cp_async_wait<0>();
     tmptx::tmem_fence_before_sync();
     __syncthreads();
@@ -935,14 +1047,6 @@ k_pass_b_rg(BatchArgs a, int ngroups) {
 }
 
 // --------------------------------------------------------------------------------------
-// k_pass_c: one block per row y; X/16 threads each own 16 pixels
-// (x = 2*(t + P*r) + h); loops over the batch keeping the per-pixel state in
-// registers.  The per-pixel sum and sum of squares are compensated (Kahan)
-// FP32 sums over the batch, added to the FP64 running sums once per batch.  At
-// X = 4096 and 2048 (128 registers, two or four blocks per SM) a thread keeps plain
-// FP32 partial sums over at most 8 orientations in registers and adds them
-// (Kahan) into compensated sums parked in its TMEM lane (columns 0-63 of its
-// 128), beside its twiddle multipliers (columns 64-127).
 // Copies of a block's shared-memory histogram: lane l counts into copy
 // l % n, bin b of copy c at word b * n + c, so that lanes of one warp whose
 // values fall in the same bin (the bins near zero take most of them) rarely
@@ -954,144 +1058,199 @@ __host__ __device__ inline int hist_copies(int bins, int max_copies) {
     return n;
 }
 
+// --------------------------------------------------------------------------------------
+// k_pass_c: the row pass.  Each row's c2r is an H = X/2-point inverse transform of the
+// even/odd packing (8 complex values = 16 pixels per thread, P = X/16 threads per
+// row); two orientations go through it side by side (tmfft::Pair), so that the
+// additions of both take one instruction, the twiddles are fetched once, the shared-memory
+// accesses are 16 bytes wide, and a thread ends with the two values of a pixel next to
+// each other: one three-way maximum and one two-wide multiply-add of the histogram.
+//
+// The transform is the Stockham plan 8, 8, ... of tmfft::fft.  Its butterflies b of stages
+// 1, 2, ... fall into 8 groups j = b mod 8 that exchange nothing after the first exchange, so
+// group j is put in G = P/8 adjacent lanes (lane l has b = 8 l + j): one exchange over the
+// whole row hands group j its P values, every later one stays in the group's part of the
+// exchange buffer (__syncwarp only).  That buffer is double, so a pair of orientations
+// costs one block barrier instead of twelve, and the warps may run almost a whole pair apart.
+// A block has max(1, 128 / P) rows, so that it is made of whole warps in every lane
+// quadrant, and goes through the image in steps of the grid (all blocks resident): twiddles
+// and histogram are set up once, and the rows of C of the next pair -- the next rows' first
+// pair after the last -- arrive by tensor-map copies while a pair is transformed.
+//
+// The per-pixel sum and sum of squares are plain FP32 sums over at most 8
+// orientations in registers, added (Kahan) every 8 orientations into
+// compensated FP32 sums in the thread's TMEM columns 0-63 and from there to the
+// FP64 running sums once per batch.  Columns 64-127 hold the thread's twiddle
+// multipliers.  The best orientation is written to memory when a pixel's
+// maximum changes (the n-th orientation changes it with probability 1/n) and never read.
 template <int X>
 struct PassC {
     static constexpr int H = X / 2;
-    static constexpr int R = 8;
-    static constexpr int P = H / R;                 // X/16 threads
-    static constexpr int RSF = tmfft::padded_len(H);
-    // X = 4096 (256 threads, two blocks per SM) and X = 2048 (128 threads, four
-    // blocks per SM): every block's warps cover the four TMEM lane quadrants, and
-    // the blocks of an SM together take its 512 columns
-    static constexpr bool COMP_IN_TMEM = (X == 4096 || X == 2048) && P % 32 == 0;
-    static constexpr int MIN_BLOCKS = X == 2048 ? 4 : 2;
-    // with the compensation terms in TMEM, a thread also keeps its twiddle
-    // multipliers there (the c2r packing's 8 and the transform's stages 1-3):
-    // 128 columns per warp, columns 0-47 sums, 48-63 packing, 64 + 16 (s - 1) stage s
-    static constexpr int WCOLS = COMP_IN_TMEM ? 128 : 64;
-    static constexpr uint32_t TMEM_COLS = WCOLS * ((P / 32 + 3) / 4);   // warps of a lane quadrant side by side
-    // one histogram copy: measured at X = 4096, 16 lane-striped copies (32 KB
-    // more shared memory per block, less L1) made this pass 5 % slower
-    static constexpr int HIST_COPIES = 1;
-    // dynamic shared memory for a row pitch XP and `bins` histogram bins
+    using PL = tmfft::Plan<H, 8>;
+    static constexpr int P = H / 8;                 // threads per row
+    static constexpr int G = P / 8;                 // lanes per group
+    static constexpr int S = P + P / 8;             // pairs of a group's part of the exchange buffer (one spare per 8)
+    static constexpr int ROWS = P >= 128 ? 1 : 128 / P;
+    static constexpr int NT = P * ROWS;             // 128 threads (256 at X = 4096)
+    static constexpr int EXL = 8 * S;               // exchange buffer of a row
+    // 512 threads per SM at 128 registers: every block has its 128 TMEM columns per warp
+    static constexpr int MIN_BLOCKS = 512 / NT;
+    static constexpr int WCOLS = 128;
+    static constexpr uint32_t TMEM_COLS = WCOLS * ((NT / 32 + 3) / 4);   // warps of a lane quadrant side by side
+    static_assert(PL::radix(0) == 8 && PL::radix(1) == 8 && (PL::stages == 3 || PL::stages == 4) && G <= 32, "pass C widths");
+    // dynamic shared memory for a row pitch XP and `bins` histogram bins (one word for values outside)
     static size_t smem_bytes(int XP, int bins) {
-        return 128 + sizeof(float2) * (2 * (size_t)XP + RSF) + 4 * (size_t)bins * hist_copies(bins, HIST_COPIES);
+        return 128 + sizeof(float2) * (size_t)ROWS * 2 * c_row_len(XP) + sizeof(float4) * 2 * (size_t)ROWS * EXL + 4 * ((size_t)bins + 1);
     }
 };
 
-// Stage multipliers of pass C's H-point inverse transform (8 values per thread),
-// parked in the thread's TMEM columns 64 + 16 (s - 1) for stage s: the R/RS
-// butterflies' RS - 1 powers each, as float pairs (tmfft::fft_pre's source).
-template <int H>
-struct PassCStageTw {
-    using PL = tmfft::Plan<H, 8>;
-    static_assert(PL::stages <= 4, "three twiddled stages fit columns 64-111");
-    uint32_t col64;
-    float tb[16];
+// the larger of three values; a NaN never wins
+__device__ __forceinline__ float fmax3(float a, float b, float c) {
+    float r;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+
+// Twiddle multipliers of stage s of the row pass's transform in lane l of group j, in 16 TMEM
+// columns: butterfly u's powers w^1 .. w^(RS-1) at float pairs u (RS - 1) + r - 1.  At
+// widths from 2048 each power is a table entry, below the product tree of
+// tmfft::apply_twiddles.
+template <int X>
+struct PassCTw {
+    using PC = PassC<X>;
+    using PL = typename PC::PL;
     template <int s>
-    __device__ __forceinline__ void issue() { tmptx::tmem_ld16(col64 + 16 * (s - 1), tb); }
-    template <int s>
-    __device__ __forceinline__ void get(int u, float2* p) {
-        constexpr int RS = PL::radix(s);
-        if (u == 0) tmptx::tmem_wait_ld16(tb);
+    __device__ static void fill(uint32_t col, int l, int j, const tmfft::Twiddles& tw) {
+        constexpr int RS = PL::radix(s), Ns = PL::ns(s), H = PC::H;
+        float g[16];
 #pragma unroll
-        for (int r = 1; r < RS; r++) p[r] = make_float2(tb[2 * (u * (RS - 1) + r - 1)], tb[2 * (u * (RS - 1) + r - 1) + 1]);
-    }
-    // the multipliers of thread t, from the twiddle table, into its columns
-    __device__ static void fill(uint32_t col64, int t, const tmfft::Twiddles& tw) {
-        tmfft::sfor<PL::stages>([&](auto sc) {
-            constexpr int s = decltype(sc)::value;
-            if constexpr (s > 0) {
-                constexpr int RS = PL::radix(s), Ns = PL::ns(s), R = 8, P = PL::P;
-                float g[16];
+        for (int i = 0; i < 16; i++) g[i] = 0.f;
 #pragma unroll
-                for (int i = 0; i < 16; i++) g[i] = 0.f;
+        for (int u = 0; u < 8 / RS; u++) {
+            const int jm = (8 * (l + PC::G * u) + j) % Ns;
+            float2 p[8];
+            if constexpr (X >= 2048) {
 #pragma unroll
-                for (int u = 0; u < R / RS; u++) {
-                    const int jm = (t + P * u) % Ns;
-#pragma unroll
-                    for (int r = 1; r < RS; r++) {
-                        const float2 w = tw.template w<+1>(jm * (H / (Ns * RS)) * r, H);
-                        g[2 * (u * (RS - 1) + r - 1)] = w.x;
-                        g[2 * (u * (RS - 1) + r - 1) + 1] = w.y;
-                    }
+                for (int r = 1; r < RS; r++) p[r] = tw.template w<+1>(jm * (H / (Ns * RS)) * r, H);
+            } else {
+                p[1] = tw.template w<+1>(jm * (H / (Ns * RS)), H);
+                if constexpr (RS > 2) { p[2] = cmul(p[1], p[1]); p[3] = cmul(p[2], p[1]); }
+                if constexpr (RS > 4) {
+                    p[4] = cmul(p[2], p[2]);
+                    p[5] = cmul(p[4], p[1]);
+                    p[6] = cmul(p[4], p[2]);
+                    p[7] = cmul(p[4], p[3]);
                 }
-                tmptx::tmem_st16(col64 + 16 * (s - 1), g);
             }
-        });
+#pragma unroll
+            for (int r = 1; r < RS; r++) {
+                g[2 * (u * (RS - 1) + r - 1)] = p[r].x;
+                g[2 * (u * (RS - 1) + r - 1) + 1] = p[r].y;
+            }
+        }
+        tmptx::tmem_st16(col, g);
+    }
+    // the stage's butterflies on v (tb: its multipliers, loaded before)
+    template <int s>
+    __device__ static __forceinline__ void stage(tmfft::Pair (&v)[8], float (&tb)[16]) {
+        constexpr int RS = PL::radix(s), NU = 8 / RS;
+        tmptx::tmem_wait_ld16(tb);
+#pragma unroll
+        for (int u = 0; u < NU; u++) {
+            tmfft::Pair e[RS];
+            e[0] = v[u];
+#pragma unroll
+            for (int r = 1; r < RS; r++) {
+                const int i = u * (RS - 1) + r - 1;
+                e[r] = tmfft::pmul(v[u + r * NU], make_float2(tb[2 * i], tb[2 * i + 1]));
+            }
+            tmfft::pdft<RS, +1>(e);
+#pragma unroll
+            for (int r = 0; r < RS; r++) v[u + r * NU] = e[r];
+        }
     }
 };
 
 template <int X>
-__global__ void __launch_bounds__(X / 16, PassC<X>::MIN_BLOCKS)
-k_pass_c(BatchArgs a, int Y) {
+__global__ void __launch_bounds__(PassC<X>::NT, PassC<X>::MIN_BLOCKS)
+k_pass_c(BatchArgs a, const __grid_constant__ CUtensorMap cmap, int Y) {
     using PC = PassC<X>;
-    constexpr int H = PC::H, P = PC::P;
-    constexpr bool kTm = PC::COMP_IN_TMEM;
-    static_assert(!kTm || PC::TMEM_COLS <= 256, "pass C TMEM columns");
+    using PL = typename PC::PL;
+    using TW = PassCTw<X>;
+    constexpr int P = PC::P, G = PC::G, S = PC::S, NT = PC::NT, ROWS = PC::ROWS, EXL = PC::EXL, H = PC::H;
     constexpr uint32_t kWaitLimit = 1u << 24;
-    const int XP = a.XP;
-    // rows of C stream in through 1-D bulk copies, double buffered: the copy
-    // of orientation o+1 runs while orientation o is transformed.
-    // dynamic shared memory: mbarriers | row buffer 0 | row buffer 1 | FFT buffer | histogram
+    const int LR = c_row_len(a.XP);   // float2 of a row in shared memory
+    // dynamic shared memory: mbarrier, TMEM slot | row pair | exchange 0 | exchange 1 | histogram
     extern __shared__ __align__(128) unsigned char smem_c[];
     uint64_t* mbar = reinterpret_cast<uint64_t*>(smem_c);
-    float2* const rows = reinterpret_cast<float2*>(smem_c + 128);   // two buffers of XP
-    float2* fbuf = rows + 2 * XP;
-    unsigned int* shist = reinterpret_cast<unsigned int*>(fbuf + PC::RSF);
-    const int t = threadIdx.x;
-    const int y = blockIdx.x;
-    const uint32_t row_bytes = (uint32_t)XP * (uint32_t)sizeof(float2);
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem_c + 64);
-    const int warp = t >> 5;
-    if (t == 0) {
-        tmptx::mbar_init(&mbar[0], 1);
-        tmptx::mbar_init(&mbar[1], 1);
+    float2* const rows = reinterpret_cast<float2*>(smem_c + 128);
+    float4* const exch = reinterpret_cast<float4*>(rows + ROWS * 2 * LR);
+    unsigned int* const shist = reinterpret_cast<unsigned int*>(exch + 2 * ROWS * EXL);
+    const int tid = threadIdx.x, warp = tid >> 5;
+    const int t = tid % P, rl = tid / P;
+    const int l = t % G, j = t / G;   // lane and group of the stages after the first
+    const int npairs = (a.nb + 1) >> 1, nblocks = Y / ROWS;
+    if (tid == 0) tmptx::mbar_init(mbar, 1);
+    if (warp == 0) {
+        tmptx::tmem_alloc(tmem_slot, PC::TMEM_COLS);
+        tmptx::tmem_relinquish();
     }
-    if constexpr (kTm) {
-        if (warp == 0) {
-            tmptx::tmem_alloc(tmem_slot, PC::TMEM_COLS);
-            tmptx::tmem_relinquish();
-        }
-    }
-    const int hcopies = hist_copies(a.hist_bins, PC::HIST_COPIES);
-    const int hcopy = t & (hcopies - 1);
-    for (int b = t; b < a.hist_bins * hcopies; b += P) shist[b] = 0u;
-    if constexpr (kTm) tmptx::tmem_fence_before_sync();
+    for (int b = tid; b <= a.hist_bins; b += NT) shist[b] = 0u;
+    tmptx::tmem_fence_before_sync();
     __syncthreads();
-    if constexpr (kTm) tmptx::tmem_fence_after_sync();
+    tmptx::tmem_fence_after_sync();
     // this thread's TMEM columns (lane quadrant warp % 4)
-    const uint32_t tcomp = kTm ? *tmem_slot + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)(PC::WCOLS * (warp >> 2)) : 0u;
-    if (t == 0 && a.nb > 0) {
-        tmptx::mbar_arrive_expect_tx(&mbar[0], row_bytes);
-        tmptx::bulk_g2s(rows, a.C + (size_t)y * XP, row_bytes, &mbar[0]);
-    }
-    float mip[16];
-    int best[16];
-    // per-pixel sum and sum of squares over the batch: compensated (Kahan) FP32,
-    // added to the FP64 running sums once per batch.  Without TMEM: fs, fq_regs
-    // and the compensation terms comp_regs[0..15] / [16..31] in registers, updated
-    // per orientation.  With TMEM (X = 4096): fs and pq are plain FP32 partial sums
-    // over at most 8 orientations, added every 8 orientations (Kahan) into the
-    // compensated sums held in TMEM columns 0-15 (sum), 16-31 (its compensation),
-    // 32-47 (sum of squares), 48-63 (its compensation).
-    float fs[16];
-    float fq_regs[kTm ? 1 : 16];
-    float pq[kTm ? 16 : 1];
-    const size_t rowoff = (size_t)y * X;
+    const uint32_t tcomp = *tmem_slot + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)(PC::WCOLS * (warp >> 2));
+    // rows rb ROWS .. of orientations 2 i and 2 i + 1 (the last of an odd batch twice), each
+    // as its column groups' pieces of the tiles (groups beyond the pitch arrive as zeros)
+    // (called by warp 0: a lane issues one box)
+    const int tile_rows = c_tile_rows(Y), boxes = c_row_boxes(a.XP), box = c_row_box(a.XP);
+    auto issue_pair = [&](int rb, int i) {
+        if (tid == 0) tmptx::mbar_arrive_expect_tx(mbar, (uint32_t)(2 * ROWS * LR) * (uint32_t)sizeof(float2));
+        __syncwarp();
+        for (int e = tid; e < 2 * ROWS * boxes; e += 32) {
+            const int k = e / (2 * ROWS), hr = e % (2 * ROWS);   // box; orientation and row
+            const int o = 2 * i + hr / ROWS, y = rb * ROWS + hr % ROWS;
+            tmptx::tensor5_g2s(rows + hr * LR + 4 * k * box, &cmap, 0, y % tile_rows, k * box, y / tile_rows,
+                               o < a.nb ? o : 2 * i, mbar);
+        }
+    };
+    if (warp == 0 && npairs > 0 && (int)blockIdx.x < nblocks) issue_pair(blockIdx.x, 0);
+    {
+        // the packing's multipliers W_X^k, k = t + P r (columns 64-79), and those of stages 1, 2, 3
+        float z[16];
 #pragma unroll
-    for (int r = 0; r < 8; r++) {
-        const int x = 2 * (t + P * r);
-        const float2 mv = *reinterpret_cast<const float2*>(a.mip + rowoff + x);
-        const int2 bv = *reinterpret_cast<const int2*>(a.best + rowoff + x);
-        mip[2 * r] = mv.x; mip[2 * r + 1] = mv.y;
-        best[2 * r] = bv.x; best[2 * r + 1] = bv.y;
-        fs[2 * r] = 0.f; fs[2 * r + 1] = 0.f;
-        if constexpr (kTm) { pq[2 * r] = 0.f; pq[2 * r + 1] = 0.f; }
+        for (int r = 0; r < 8; r++) {
+            const float2 w = a.tw.template w<+1>(t + P * r, X);
+            z[2 * r] = w.x;
+            z[2 * r + 1] = w.y;
+        }
+        tmptx::tmem_st16(tcomp + 64, z);
+        TW::template fill<1>(tcomp + 80, l, j, a.tw);
+        TW::template fill<2>(tcomp + 96, l, j, a.tw);
+        if constexpr (PL::stages == 4) TW::template fill<3>(tcomp + 112, l, j, a.tw);
+        tmptx::tmem_wait_st();
     }
-    // the compensation terms: in registers, or parked in TMEM between orientations
-    float comp_regs[kTm ? 1 : 32];
-    if constexpr (kTm) {
+    // value v[r] holds the pixels own + 2 P r (real parts) and the next (imaginary parts)
+    const int own = rl * X + 16 * l + 2 * j;
+    // histogram bin int((v - min) / step) as one multiply-add: (v - min) / step = v / step + hoff
+    const float hoff = -a.hist_min * a.hist_inv_step;
+    const float2 hinv2 = make_float2(a.hist_inv_step, a.hist_inv_step), hoff2 = make_float2(hoff, hoff);
+    const unsigned int nbins = (unsigned int)a.hist_bins;
+    bool timed_out = false, stop = false;
+    uint32_t n = 0;   // pairs done: parity of the barrier's phase and of the exchange buffer
+    for (int rb = blockIdx.x; rb < nblocks && !stop; rb += gridDim.x) {
+    const size_t pix0 = (size_t)rb * ROWS * X;
+    float mip[16];
+    float fs[16], pq[16];   // plain sums over at most 8 orientations
+#pragma unroll
+    for (int r = 0; r < 16; r++) {
+        mip[r] = a.mip[pix0 + own + 2 * P * (r / 2) + r % 2];
+        fs[r] = 0.f;
+        pq[r] = 0.f;
+    }
+    {
         float z[16];
 #pragma unroll
         for (int i = 0; i < 16; i++) z[i] = 0.f;
@@ -1099,191 +1258,205 @@ k_pass_c(BatchArgs a, int Y) {
         tmptx::tmem_st16(tcomp + 16, z);
         tmptx::tmem_st16(tcomp + 32, z);
         tmptx::tmem_st16(tcomp + 48, z);
-        // the packing's multipliers W_X^k, k = t + P r (columns 112-127), and the
-        // transform's stage multipliers (64-111)
-#pragma unroll
-        for (int r = 0; r < 8; r++) {
-            const float2 w = a.tw.template w<+1>(t + P * r, X);
-            z[2 * r] = w.x;
-            z[2 * r + 1] = w.y;
-        }
-        tmptx::tmem_st16(tcomp + 112, z);
-        PassCStageTw<H>::fill(tcomp + 64, t, a.tw);
         tmptx::tmem_wait_st();
-    } else {
-#pragma unroll
-        for (int i = 0; i < (kTm ? 1 : 32); i++) comp_regs[i] = 0.f;
-#pragma unroll
-        for (int i = 0; i < (kTm ? 1 : 16); i++) fq_regs[i] = 0.f;
     }
-    auto sync = [] __device__() { __syncthreads(); };
-    // histogram bin int((v - min) / step) as one multiply-add: (v - min) / step = v / step + hoff
-    const float hoff = -a.hist_min * a.hist_inv_step;
-    // Copy o goes to buffer o & 1 and completes phase o >> 1 of that buffer's
-    // mbarrier.  After a wait runs out the block stops issuing copies and, before
-    // it exits, waits for the copies still in flight at the parity of the phase
-    // each one completes (bounded again).
-    auto drain = [&](int o) {
-        tmptx::mbar_wait_bounded(&mbar[(o - 1) & 1], ((o - 1) >> 1) & 1, kWaitLimit);   // the wait that ran out
-        if (o < a.nb) tmptx::mbar_wait_bounded(&mbar[o & 1], (o >> 1) & 1, kWaitLimit);   // issued at o - 1
-    };
-    bool timed_out = false;
-    int o = 0;
-    for (; o < a.nb; o++) {
-        const int buf = o & 1;
-        // iteration o-1 is done with row buffer buf ^ 1; every thread learns whether a wait ran out
-        if (__syncthreads_or(timed_out)) break;
-        if (t == 0 && o + 1 < a.nb) {
-            tmptx::mbar_arrive_expect_tx(&mbar[buf ^ 1], row_bytes);
-            tmptx::bulk_g2s(rows + (buf ^ 1) * XP, a.C + ((size_t)(o + 1) * Y + y) * XP, row_bytes, &mbar[buf ^ 1]);
-        }
-        float pk[kTm ? 16 : 1];   // the packing's multipliers, from TMEM
-        if constexpr (kTm) tmptx::tmem_ld16(tcomp + 112, pk);
-        if (!tmptx::mbar_wait_bounded(&mbar[buf], (o >> 1) & 1, kWaitLimit)) {
+    for (int i = 0; i < npairs; i++, n++) {
+        float4* const ex = exch + (n & 1) * (ROWS * EXL) + rl * EXL;
+        float tb[16];
+        tmptx::tmem_ld16(tcomp + 64, tb);
+        if (!tmptx::mbar_wait_bounded(mbar, n & 1, kWaitLimit)) {
             timed_out = true;
             atomicExch(a.err, 1);
         }
-        if constexpr (kTm) tmptx::tmem_wait_ld16(pk);
-        const float2* rb = rows + buf * XP;
-        float2 v[8];
+        tmfft::Pair v[8];
+        tmptx::tmem_wait_ld16(tb);
+        {
+            const float2* c = rows + rl * LR + t;
+            const float2* d = rows + rl * LR + (P - t);
 #pragma unroll
-        for (int r = 0; r < 8; r++) {
-            const int k = t + P * r;
-            float2 hk = rb[k];
-            float2 hm = rb[H - k];
-            if (k == 0) { hk.y = 0.f; hm.y = 0.f; }
-            const float2 e = make_float2(hk.x + hm.x, hk.y - hm.y);
-            const float2 d = make_float2(hk.x - hm.x, hk.y + hm.y);
-            const float2 od = cmul(d, kTm ? make_float2(pk[2 * r], pk[2 * r + 1]) : a.tw.template w<+1>(k, X));
-            v[r] = make_float2(e.x - od.y, e.y + od.x);
-        }
-        // the barrier at the top of the iteration follows the last reads of fbuf
-        if constexpr (kTm) {
-            PassCStageTw<H> stw{tcomp + 64, {}};
-            tmfft::fft_pre<H, 8, +1, false>(v, t, fbuf, stw, sync);
-        } else {
-            tmfft::fft<H, 8, +1, false>(v, t, fbuf, a.tw, sync);
-        }
-        const int g = (int)(a.gidx0 + o);
-        if constexpr (kTm) {
-            // MIP / argmax, histogram and the plain partial sums of this orientation
-#pragma unroll
-            for (int r = 0; r < 8; r++) {
+            for (int r = 0; r < 8; r++) {   // k = t + P r and H - k
+                const float2 w = make_float2(tb[2 * r], tb[2 * r + 1]);
+                float2 z[2];
 #pragma unroll
                 for (int h = 0; h < 2; h++) {
-                    const float val = h ? v[r].y : v[r].x;
-                    const int pi = 2 * r + h;
-                    if (val > mip[pi]) { mip[pi] = val; best[pi] = g; }
-                    fs[pi] += val;
-                    pq[pi] = fmaf(val, val, pq[pi]);
-                    const int bin = __float2int_rz(fmaf(val, a.hist_inv_step, hoff));
-                    if ((unsigned)bin < (unsigned)a.hist_bins) atomicAdd(&shist[bin * hcopies + hcopy], 1u);
+                    float2 hk = c[h * ROWS * LR + P * r], hm = d[h * ROWS * LR + P * (7 - r)];
+                    if (r == 0 && t == 0) hk.y = hm.y = 0.f;   // as FFTW's c2r
+                    const float2 e = make_float2(hk.x + hm.x, hk.y - hm.y);
+                    const float2 df = make_float2(hk.x - hm.x, hk.y + hm.y);
+                    const float2 od = cmul(df, w);
+                    z[h] = make_float2(e.x - od.y, e.y + od.x);
                 }
-            }
-            if ((o & 7) == 7 || o == a.nb - 1) {
-                // Kahan: the compensation holds what the last addition added beyond its input
-#pragma unroll
-                for (int sweep = 0; sweep < 4; sweep++) {   // 8 pixels of one sum at a time
-                    float* part = ((sweep >> 1) ? pq : fs) + 8 * (sweep & 1);
-                    const uint32_t col = tcomp + 32 * (sweep >> 1) + 8 * (sweep & 1);
-                    float sm[8], cm[8];   // sum, compensation
-                    tmptx::tmem_ld8(col, sm);
-                    tmptx::tmem_ld8(col + 16, cm);
-                    tmptx::tmem_wait_ld8x2(sm, cm);
-#pragma unroll
-                    for (int i = 0; i < 8; i++) {
-                        const float yv = part[i] - cm[i];
-                        const float tv = sm[i] + yv;
-                        cm[i] = (tv - sm[i]) - yv;
-                        sm[i] = tv;
-                        part[i] = 0.f;
-                    }
-                    tmptx::tmem_st8(col, sm);
-                    tmptx::tmem_st8(col + 16, cm);
-                }
-                tmptx::tmem_wait_st();
-            }
-        } else {
-            // epilogue in two sweeps over the 16 values, so that only one sum's 16
-            // compensation terms are live at a time: (1) MIP / argmax, histogram and
-            // the sum, (2) the sum of squares
-#pragma unroll
-            for (int sweep = 0; sweep < 2; sweep++) {
-                float* comp = comp_regs + 16 * sweep;
-#pragma unroll
-                for (int r = 0; r < 8; r++) {
-#pragma unroll
-                    for (int h = 0; h < 2; h++) {
-                        const float val = h ? v[r].y : v[r].x;
-                        const int pi = 2 * r + h;
-                        // Kahan: the compensation holds what the last addition added beyond its input
-                        if (sweep == 0) {
-                            if (val > mip[pi]) { mip[pi] = val; best[pi] = g; }
-                            const float ys = val - comp[pi];
-                            const float ts = fs[pi] + ys;
-                            comp[pi] = (ts - fs[pi]) - ys;
-                            fs[pi] = ts;
-                            const int bin = __float2int_rz(fmaf(val, a.hist_inv_step, hoff));
-                            if ((unsigned)bin < (unsigned)a.hist_bins) atomicAdd(&shist[bin * hcopies + hcopy], 1u);
-                        } else {
-                            const float yq = fmaf(val, val, -comp[pi]);
-                            const float tq = fq_regs[pi] + yq;
-                            comp[pi] = (tq - fq_regs[pi]) - yq;
-                            fq_regs[pi] = tq;
-                        }
-                    }
-                }
+                v[r] = {make_float2(z[0].x, z[1].x), make_float2(z[0].y, z[1].y)};
             }
         }
+        auto put = [](float4* at, tmfft::Pair p) { *at = make_float4(p.re.x, p.re.y, p.im.x, p.im.y); };
+        auto get = [](const float4* at) {
+            const float4 f = *at;
+            return tmfft::Pair{make_float2(f.x, f.y), make_float2(f.z, f.w)};
+        };
+        tmfft::pdft<8, +1>(v);
+#pragma unroll
+        for (int r = 0; r < 8; r++) put(ex + S * r + t, v[r]);
+        tmptx::tmem_ld16(tcomp + 80, tb);
+        if (__syncthreads_or(timed_out)) {   // every thread learns whether a wait ran out
+            stop = true;
+            break;
+        }
+        // every thread has read its row values: the next pair's rows may arrive
+        if (warp == 0) {
+            if (i + 1 < npairs) issue_pair(rb, i + 1);
+            else if (rb + (int)gridDim.x < nblocks) issue_pair(rb + gridDim.x, 0);
+        }
+        float4* const eg = ex + S * j;
+#pragma unroll
+        for (int r = 0; r < 8; r++) v[r] = get(eg + l + G * r);
+        TW::template stage<1>(v, tb);
+        tmptx::tmem_ld16(tcomp + 96, tb);
+        auto pad = [](int e) { return e + (e >> 3); };
+        __syncwarp();   // the group's values are read
+#pragma unroll
+        for (int r = 0; r < 8; r++) put(eg + 9 * l + r, v[r]);   // pad(8 l + r)
+        __syncwarp();
+#pragma unroll
+        for (int r = 0; r < 8; r++) v[r] = get(eg + pad(l + G * r));
+        TW::template stage<2>(v, tb);
+        if constexpr (PL::stages == 4) {
+            tmptx::tmem_ld16(tcomp + 112, tb);
+            __syncwarp();
+            const int at = 72 * (l >> 3) + (l & 7);
+#pragma unroll
+            for (int r = 0; r < 8; r++) put(eg + at + 9 * r, v[r]);   // pad(64 (l / 8) + l % 8 + 8 r)
+            __syncwarp();
+#pragma unroll
+            for (int r = 0; r < 8; r++) v[r] = get(eg + pad(l + G * r));
+            TW::template stage<3>(v, tb);
+        }
+        // values of orientations 2 i and 2 i + 1 at the thread's pixel r
+        auto val = [&](int r) { return r % 2 ? v[r / 2].im : v[r / 2].re; };
+        const int g = (int)a.gidx0 + 2 * i;
+        const bool two = 2 * i + 1 < a.nb;   // else the second repeats the first
+#pragma unroll
+        for (int r0 = 0; r0 < 16; r0 += 4) {
+            // strict >, first orientation first: the new maximum is v.x, else v.y, else the old one
+            float m[4];
+            bool changed = false;
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                m[k] = fmax3(mip[r0 + k], val(r0 + k).x, val(r0 + k).y);
+                changed = changed || m[k] > mip[r0 + k];
+            }
+            if (changed) {
+#pragma unroll
+                for (int k = 0; k < 4; k++)
+                    if (m[k] > mip[r0 + k]) a.best[pix0 + own + 2 * P * ((r0 + k) / 2) + k % 2] = val(r0 + k).x == m[k] ? g : g + 1;
+            }
+#pragma unroll
+            for (int k = 0; k < 4; k++) mip[r0 + k] = m[k];
+        }
+        auto count = [&](float b) {
+            const unsigned int bin = (unsigned int)__float2int_rz(b);
+            atomicAdd(&shist[bin < nbins ? bin : nbins], 1u);
+        };
+        if (two) {
+#pragma unroll
+            for (int r = 0; r < 16; r++) {
+                const float2 p = val(r);
+                fs[r] += p.x;
+                pq[r] = fmaf(p.x, p.x, pq[r]);
+                fs[r] += p.y;
+                pq[r] = fmaf(p.y, p.y, pq[r]);
+                const float2 b = tmfft::fma2(p, hinv2, hoff2);
+                count(b.x);
+                count(b.y);
+            }
+        } else {
+#pragma unroll
+            for (int r = 0; r < 16; r++) {
+                const float p = val(r).x;
+                fs[r] += p;
+                pq[r] = fmaf(p, p, pq[r]);
+                count(fmaf(p, a.hist_inv_step, hoff));
+            }
+        }
+        if ((i & 3) == 3 || i == npairs - 1) {
+            // Kahan: the compensation holds what the last addition added beyond its input
+#pragma unroll
+            for (int sweep = 0; sweep < 4; sweep++) {   // 8 pixels of one sum at a time
+                float* part = ((sweep >> 1) ? pq : fs) + 8 * (sweep & 1);
+                const uint32_t col = tcomp + 32 * (sweep >> 1) + 8 * (sweep & 1);
+                float sm[8], cm[8];   // sum, compensation
+                tmptx::tmem_ld8(col, sm);
+                tmptx::tmem_ld8(col + 16, cm);
+                tmptx::tmem_wait_ld8x2(sm, cm);
+#pragma unroll
+                for (int k = 0; k < 8; k++) {
+                    const float yv = part[k] - cm[k];
+                    const float tv = sm[k] + yv;
+                    cm[k] = (tv - sm[k]) - yv;
+                    sm[k] = tv;
+                    part[k] = 0.f;
+                }
+                tmptx::tmem_st8(col, sm);
+                tmptx::tmem_st8(col + 16, cm);
+            }
+            tmptx::tmem_wait_st();
+        }
     }
-    // the sums and their compensation terms for the FP64 flush
-    float send[kTm ? 64 : 1];
-    const float* fsend = fs;
-    const float* cend = comp_regs;
-    const float* fqend = fq_regs;
-    const float* cqend = comp_regs + (kTm ? 0 : 16);
-    if constexpr (kTm) {
+    if (stop) break;
+    // the batch's sums into the FP64 running sums, and the maxima, in pixel order through the
+    // exchange buffers (one spare element per 16: the strided writes are conflict-free), so that
+    // memory is accessed in whole lines with all of a thread's loads in flight
+    double* const staged = reinterpret_cast<double*>(exch);
+    auto pad = [](int e) { return e + (e >> 4); };
+    const int at = pad(own);
+    auto px = [pad](int r) { return pad(2 * P * (r / 2)) + r % 2; };
+    constexpr int PER = ROWS * X / NT;   // 16
+    __syncthreads();   // every group is done with its transposes
+    {
+        float send[32];
         tmptx::tmem_ld16(tcomp, send);
         tmptx::tmem_ld16(tcomp + 16, send + 16);
         tmptx::tmem_wait_ld32(send);
-        tmptx::tmem_ld16(tcomp + 32, send + 32);
-        tmptx::tmem_ld16(tcomp + 48, send + 48);
-        tmptx::tmem_wait_ld32(send + 32);
-        fsend = send;
-        cend = send + 16;
-        fqend = send + 32;
-        cqend = send + 48;
-        tmptx::tmem_fence_before_sync();
-    }
-    const bool failed = __syncthreads_or(timed_out);
-    if constexpr (kTm) {
-        // every warp has finished with its TMEM columns (the barrier above)
-        tmptx::tmem_fence_after_sync();
-        if (warp == 0) tmptx::tmem_dealloc(*tmem_slot, PC::TMEM_COLS);
-    }
-    if (failed) {
-        // results of this block are discarded (the host reports the timeout)
-        drain(o);
-        return;
-    }
 #pragma unroll
-    for (int r = 0; r < 8; r++) {
-        const int x = 2 * (t + P * r);
-        *reinterpret_cast<float2*>(a.mip + rowoff + x) = make_float2(mip[2 * r], mip[2 * r + 1]);
-        *reinterpret_cast<int2*>(a.best + rowoff + x) = make_int2(best[2 * r], best[2 * r + 1]);
-        double2 sv = *reinterpret_cast<const double2*>(a.sum + rowoff + x);
-        double2 qv = *reinterpret_cast<const double2*>(a.sumsq + rowoff + x);
-        sv.x += (double)fsend[2 * r] - (double)cend[2 * r];
-        sv.y += (double)fsend[2 * r + 1] - (double)cend[2 * r + 1];
-        qv.x += (double)fqend[2 * r] - (double)cqend[2 * r];
-        qv.y += (double)fqend[2 * r + 1] - (double)cqend[2 * r + 1];
-        *reinterpret_cast<double2*>(a.sum + rowoff + x) = sv;
-        *reinterpret_cast<double2*>(a.sumsq + rowoff + x) = qv;
+        for (int r = 0; r < 16; r++) staged[at + px(r)] = (double)send[r] - (double)send[16 + r];
+        tmptx::tmem_ld16(tcomp + 32, send);
+        tmptx::tmem_ld16(tcomp + 48, send + 16);
+        tmptx::tmem_wait_ld32(send);
+#pragma unroll
+        for (int r = 0; r < 16; r++) staged[2 * ROWS * EXL + at + px(r)] = (double)send[r] - (double)send[16 + r];
     }
     __syncthreads();
-    for (int b = t; b < a.hist_bins; b += P) {
-        unsigned int cnt = 0;
-        for (int k = 0; k < hcopies; k++) cnt += shist[b * hcopies + k];
+#pragma unroll 1
+    for (int k = 0; k < 2; k++) {
+        double* const dst = (k ? a.sumsq : a.sum) + pix0 + tid;
+        double d[PER];
+#pragma unroll
+        for (int e = 0; e < PER; e++) d[e] = dst[e * NT];
+#pragma unroll
+        for (int e = 0; e < PER; e++) dst[e * NT] = d[e] + staged[k * 2 * ROWS * EXL + pad(tid + e * NT)];
+    }
+    __syncthreads();
+    float* const stage = reinterpret_cast<float*>(exch);
+#pragma unroll
+    for (int r = 0; r < 16; r++) stage[at + px(r)] = mip[r];
+    __syncthreads();
+#pragma unroll
+    for (int e = 0; e < PER; e++) a.mip[pix0 + tid + e * NT] = stage[pad(tid + e * NT)];
+    __syncthreads();   // the exchange buffers are free again
+    }
+    tmptx::tmem_fence_before_sync();
+    __syncthreads();
+    // every warp has finished with its TMEM columns (the barrier above)
+    tmptx::tmem_fence_after_sync();
+    if (warp == 0) tmptx::tmem_dealloc(*tmem_slot, PC::TMEM_COLS);
+    if (stop) {
+        // results of these rows are discarded (the host reports the timeout).  The wait for this
+        // pair ran out and none was issued after it: wait (bounded again) for its copies
+        tmptx::mbar_wait_bounded(mbar, n & 1, kWaitLimit);
+        return;
+    }
+    for (int b = tid; b < a.hist_bins; b += NT) {
+        const unsigned int cnt = shist[b];
         if (cnt) atomicAdd(a.hist + b, (unsigned long long)cnt);
     }
 }
@@ -1323,23 +1496,64 @@ __global__ void k_reset_state(float* mip, int* best, double* sum, double* sumsq,
 }
 
 // --------------------------------------------------------------------------------------
+// The tensor maps of a correlation buffer C of `cap` orientations.
+//   rows      as the row pass reads it: dimensions (8 floats of a column group's row, row of the
+//             tile, column group, tile row, orientation), boxes of one row x c_row_box(XP)
+//             groups.  L2 promotion to 64 bytes: 0.39 ms for a load-only pass over 2.15 GB
+//             against 0.45 without and with 128 or 256 bytes.
+//   columns   as k_pass_b_rg writes it: dimensions (a tile, column group, tile row), boxes of
+//             256 tiles of one column group
+struct CMaps {
+    CUtensorMap rows, columns;
+};
+inline cudaError_t c_tensor_maps(CMaps* maps, float2* C, int XP, int Y, int cap) {
+    void* fn = nullptr;
+    cudaDriverEntryPointQueryResult found;
+    const cudaError_t e = cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &fn, 12000, cudaEnableDefault, &found);
+    if (e != cudaSuccess) return e;
+    if (found != cudaDriverEntryPointSuccess || !fn) return cudaErrorNotSupported;
+    const auto encode = reinterpret_cast<decltype(&cuTensorMapEncodeTiled)>(fn);
+    const int R = c_tile_rows(Y);
+    const cuuint32_t step[5] = {1, 1, 1, 1, 1};
+    {
+        const cuuint64_t dim[5] = {8, (cuuint64_t)R, (cuuint64_t)(XP / 4), (cuuint64_t)(Y / R), (cuuint64_t)cap};
+        const cuuint64_t stride[4] = {32, 32 * (cuuint64_t)R, (cuuint64_t)XP * 8 * R, (cuuint64_t)XP * 8 * Y};
+        const cuuint32_t box[5] = {8, 1, (cuuint32_t)c_row_box(XP), 1, 1};
+        const CUresult r = encode(&maps->rows, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 5, C, dim, stride, box, step,
+                                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                                  CU_TENSOR_MAP_L2_PROMOTION_L2_64B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+        if (r != CUDA_SUCCESS) return cudaErrorInvalidValue;
+    }
+    const cuuint64_t dim[3] = {8 * (cuuint64_t)R, (cuuint64_t)(XP / 4), (cuuint64_t)cap * (Y / R)};
+    const cuuint64_t stride[2] = {32 * (cuuint64_t)R, (cuuint64_t)XP * 8 * R};
+    const cuuint32_t box[3] = {8 * (cuuint32_t)R, 1, dim[2] < 256 ? (cuuint32_t)dim[2] : 256};
+    const CUresult r = encode(&maps->columns, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, C, dim, stride, box, step,
+                              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE,
+                              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
+}
+
+// --------------------------------------------------------------------------------------
 // Launch shapes of one geometry, shared by every entry point.
 template <int T, int X, int Y>
 struct Launch {
     using PB = PassB<T, Y>;
     using PC = PassC<X>;
+    static_assert(Y % PC::ROWS == 0, "pass C blocks hold whole groups of rows");
     using SC = SliceCol<T>;
     using RC = RowC2R<T>;
     static constexpr int pass_b_width = PB::WG;   // row pitch alignment (columns)
     // 4096-high micrographs with 256-row pruned transforms: the residue-grouped column pass
     static constexpr bool RG = (T == 256 && Y == 4096);
-    static cudaError_t configure(int XP, int bins) {
+    static cudaError_t configure_b() {
         cudaError_t e = cudaFuncSetAttribute(k_pass_b<T, Y>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PB::SMEM);
-        if (e != cudaSuccess) return e;
-        if constexpr (RG) {
+        if (RG && e == cudaSuccess)
             e = cudaFuncSetAttribute(k_pass_b_rg, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PassBRg::SMEM);
-            if (e != cudaSuccess) return e;
-        }
+        return e;
+    }
+    static cudaError_t configure(int XP, int bins) {
+        const cudaError_t e = configure_b();
+        if (e != cudaSuccess) return e;
         return cudaFuncSetAttribute(k_pass_c<X>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PC::smem_bytes(XP, bins));
     }
     // slice, projection, normalisation and row transforms
@@ -1349,15 +1563,16 @@ struct Launch {
         k_norm<T><<<(a.nb + 7) / 8, 256, 0, s>>>(a, a.norm_pixels > 0 ? a.norm_pixels : (long long)X * Y);
         k_pass_a<T, X><<<dim3(T, a.nb), X / 16, 0, s>>>(a);
     }
-    static void pass_b(BatchArgs& a, cudaStream_t s, int nsm) {
+    static void pass_b(BatchArgs& a, const CMaps& cmaps, cudaStream_t s, int nsm) {
         const int ngroups = a.XP / PB::WG;
         if (RG && ColSchedule::max_items(ngroups, a.nb, nsm) <= PassBRg::MAX_ITEMS)
-            k_pass_b_rg<<<nsm, PassBRg::NT, PassBRg::SMEM, s>>>(a, ngroups);
+            k_pass_b_rg<<<nsm, PassBRg::NT, PassBRg::SMEM, s>>>(a, cmaps.columns, ngroups);
         else
             k_pass_b<T, Y><<<nsm, PB::NT, PB::SMEM, s>>>(a, ngroups);
     }
-    static void pass_c(BatchArgs& a, cudaStream_t s) {
-        k_pass_c<X><<<Y, X / 16, PC::smem_bytes(a.XP, a.hist_bins), s>>>(a, Y);
+    static void pass_c(BatchArgs& a, const CMaps& cmaps, cudaStream_t s, int nsm) {
+        const int nblocks = Y / PC::ROWS, resident = PC::MIN_BLOCKS * nsm;
+        k_pass_c<X><<<nblocks < resident ? nblocks : resident, PC::NT, PC::smem_bytes(a.XP, a.hist_bins), s>>>(a, cmaps.rows, Y);
     }
 };
 

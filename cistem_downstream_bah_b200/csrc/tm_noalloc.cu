@@ -8,6 +8,7 @@
 // intermediate of the search lives in one file-scope device array of fixed
 // size (kScratchBytes), which each GPU that loads this library keeps until
 // the process exits.
+#include <cuda.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 #include <float.h>
@@ -82,10 +83,10 @@ struct NoAllocImpl {
     // every compiled geometry fits the fixed array (checked when this file compiles)
     static_assert(layout.total <= kScratchBytes, "a no-alloc geometry exceeds the fixed scratch array");
     static cudaError_t configure(int XP, int bins) { return LN::configure(XP, bins); }
-    static void run_batch(tmna::tmk::BatchArgs& a, cudaStream_t s, int nsm) {
+    static void run_batch(tmna::tmk::BatchArgs& a, const tmna::tmk::CMaps& cmaps, cudaStream_t s, int nsm) {
         LN::prep(a, s);
-        LN::pass_b(a, s, nsm);
-        LN::pass_c(a, s);
+        LN::pass_b(a, cmaps, s, nsm);
+        LN::pass_c(a, cmaps, s, nsm);
     }
 };
 
@@ -93,7 +94,7 @@ struct NoAllocVariant {
     int T, X, Y;
     ScratchLayout layout;
     cudaError_t (*configure)(int XP, int bins);
-    void (*run_batch)(tmna::tmk::BatchArgs&, cudaStream_t, int);
+    void (*run_batch)(tmna::tmk::BatchArgs&, const tmna::tmk::CMaps&, cudaStream_t, int);
 };
 
 #define TM_NOALLOC_VARIANT(T, X, Y) \
@@ -199,6 +200,10 @@ int run_noalloc(int device, const NoAllocVariant& var, const tm_dims* dims, cons
     a.twy = a.tw;   // the geometries here are powers of two: X, Y and T divide lmax
     a.twt = a.tw;
 
+    // C as the kernels read and write it (host work only)
+    tmna::tmk::CMaps cmaps;
+    if (tmna::tmk::c_tensor_maps(&cmaps, a.C, L.XP, Y, kBatch) != cudaSuccess) return TM_ERR_CUDA;
+
     // The array keeps the previous call's contents: rebuild the tables, clear
     // the error flag and the row spectra (their columns beyond X/2 are read as zero).
     k_noalloc_twiddles<<<(L.lmax + 255) / 256, 256, 0, s>>>(reinterpret_cast<float2*>(base + L.tw), L.lmax);
@@ -215,7 +220,7 @@ int run_noalloc(int device, const NoAllocVariant& var, const tm_dims* dims, cons
         a.nb = nb;
         a.orient0 = 0;
         a.gidx0 = (long long)first_orientation_index + b0;
-        var.run_batch(a, s, nsm);
+        var.run_batch(a, cmaps, s, nsm);
         if (cudaGetLastError() != cudaSuccess) return TM_ERR_CUDA;
     }
     int flag = 0;

@@ -3,6 +3,7 @@
 // core MMA (tcgen05.mma, kind::f16) with its shared-memory matrix descriptors.
 // No cluster multicast is used anywhere.
 #pragma once
+#include <cuda.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -48,6 +49,27 @@ __device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t by
         "l"(src), "r"(bytes), "r"(smem_u32(bar))
         : "memory");
 }
+
+// Tensor-map copy of one box global -> shared (this CTA, no multicast), completion signalled
+// on `bar`.  dst 128-byte aligned; c0 x the element size a multiple of 16.
+__device__ __forceinline__ void tensor5_g2s(void* dst, const CUtensorMap* map, int c0, int c1, int c2, int c3, int c4, uint64_t* bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.5d.shared::cta.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5, %6}], [%7];" ::"r"(
+            smem_u32(dst)),
+        "l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4), "r"(smem_u32(bar))
+        : "memory");
+}
+
+// Tensor-map store of one box shared -> global; src 128-byte aligned, no negative
+// coordinate.  Its bulk group: commit, wait until the sources have been read, until it is done.
+__device__ __forceinline__ void tensor3_s2g(const CUtensorMap* map, int c0, int c1, int c2, const void* src) {
+    asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%1, %2, %3}], [%4];" ::"l"(map), "r"(c0),
+                 "r"(c1), "r"(c2), "r"(smem_u32(src))
+                 : "memory");
+}
+__device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
+__device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 
 // Ampere-style asynchronous 8-byte copy global -> shared (LDGSTS) and its groups.
 __device__ __forceinline__ void cp_async8(void* dst, const void* src) {
