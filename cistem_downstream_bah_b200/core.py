@@ -205,7 +205,7 @@ class SearchCore:
 
     def image_results(self, image):
         n = self.X * self.Y
-        out = {k: np.zeros(n, np.float32) for k in ("mip", "psi", "theta", "phi")}
+        out = {k: np.empty(n, np.float32) for k in ("mip", "psi", "theta", "phi")}
         self._check(self.L.tm_get_image_results(self.h, int(image), _ptr(out["mip"]), _ptr(out["psi"]),
                                                 _ptr(out["theta"]), _ptr(out["phi"])))
         return out
@@ -235,9 +235,9 @@ class SearchCore:
 
     def results(self):
         n = self.X * self.Y
-        out = {k: np.zeros(n, np.float32) for k in ("mip", "psi", "theta", "phi", "defocus", "pixel")}
-        s = np.zeros(n, np.float64)
-        q = np.zeros(n, np.float64)
+        out = {k: np.empty(n, np.float32) for k in ("mip", "psi", "theta", "phi", "defocus", "pixel")}
+        s = np.empty(n, np.float64)
+        q = np.empty(n, np.float64)
         h = np.zeros(self.hist_bins, np.int64)
         self._check(self.L.tm_get_results(self.h, _ptr(out["mip"]), _ptr(out["psi"]), _ptr(out["theta"]),
                                           _ptr(out["phi"]), _ptr(out["defocus"]), _ptr(out["pixel"]),

@@ -12,6 +12,7 @@
 #include <string.h>
 
 #include <algorithm>
+#include <atomic>
 #include <chrono>
 #include <string>
 #include <thread>
@@ -40,6 +41,9 @@ struct Plane {
 
 struct Variant;
 
+constexpr int kFetchThreads = 12;
+constexpr size_t kFetchSlot = (size_t)2 << 20;   // bytes
+
 }  // namespace
 
 struct tm_ctx {
@@ -61,7 +65,9 @@ struct tm_ctx {
     double *sum = nullptr, *sumsq = nullptr;
     unsigned long long* hist = nullptr;
     int* err_flag = nullptr;
-    int* best_host = nullptr;   // page-locked copy of the best-orientation map (tm_get_results)
+    // result maps on their way to the host (fetch_parts): a page-locked slot and a stream per thread
+    char* fetch_slot[kFetchThreads] = {};
+    cudaStream_t fetch_stream[kFetchThreads] = {};
     int precision = TM_PRECISION_FP32;
     tmk::GenPlan gen_px{}, gen_py{}, gen_ph{};   // radix plans of X, Y and X/2 (sizes without compiled kernels)
     uint4* dft = nullptr;       // DFT operands of the tensor-core row pass (FP16 form)
@@ -536,7 +542,10 @@ void free_all(tm_ctx* c) {
             if (p) cudaFree(p);
     }
     c->slots.clear();
-    if (c->best_host) cudaFreeHost(c->best_host);
+    for (char* p : c->fetch_slot)
+        if (p) cudaFreeHost(p);
+    for (cudaStream_t s : c->fetch_stream)
+        if (s) cudaStreamDestroy(s);
     if (c->stream) cudaStreamDestroy(c->stream);
     cudaEvent_t evs[] = {c->ev_start, c->ev_prep, c->ev_b, c->ev_c, c->ev_end};
     for (cudaEvent_t e : evs)
@@ -544,6 +553,123 @@ void free_all(tm_ctx* c) {
     for (auto& set : c->ev_batch)
         for (cudaEvent_t e : set)
             if (e) cudaEventDestroy(e);
+}
+
+// Decodes best-orientation indices into angles and plane offsets (any output may be null).
+struct DecodeTo {
+    float *psi, *theta, *phi, *defocus, *pixel;
+};
+void decode_best(const tm_ctx* c, const int* best, size_t n, size_t at, const DecodeTo& d) {
+    const Plane* p = nullptr;   // the plane of the last index: neighbours mostly share it
+    for (size_t i = 0; i < n; i++) {
+        const int g = best[i];
+        float psi = 0, th = 0, ph = 0, df = 0, px = 0;
+        if (g >= 0) {
+            if (!p || g < p->base || g >= p->base + p->n) {
+                // planes are in increasing base order
+                auto it = std::upper_bound(c->planes.begin(), c->planes.end(), (long long)g,
+                                           [](long long v, const Plane& q) { return v < q.base; });
+                p = it == c->planes.begin() ? nullptr : &*(it - 1);
+                if (p && g >= p->base + p->n) p = nullptr;
+            }
+            if (p) {
+                const float* ang = c->angle_lists[p->angles_id].data() + 3 * (size_t)(g - p->base);
+                ph = ang[0];
+                th = ang[1];
+                psi = ang[2];
+                df = p->defocus;
+                px = p->pixel;
+            }
+        }
+        if (d.psi) d.psi[at + i] = psi;
+        if (d.theta) d.theta[at + i] = th;
+        if (d.phi) d.phi[at + i] = ph;
+        if (d.defocus) d.defocus[at + i] = df;
+        if (d.pixel) d.pixel[at + i] = px;
+    }
+}
+
+// Copies device arrays to host memory (or decodes them there).  The copies go in pieces
+// through page-locked slots, each by a thread that then moves its piece into the caller's memory:
+// that memory is usually fresh, and its page faults, one thread's work in a plain cudaMemcpy,
+// are most of the time (4096 x 4096 results, 671 MB of maps: 80-95 ms with plain copies).
+// Little data stays on the calling thread, as starting threads costs more there (256 x 256: 1.8
+// ms with 16 threads).
+struct FetchPart {
+    const void* src;      // device
+    size_t bytes;
+    char* dst;            // null: best-orientation indices to decode
+};
+int fetch_parts(tm_ctx* c, const std::vector<FetchPart>& parts, const DecodeTo& to) {
+    struct Piece {
+        int part;
+        size_t off, bytes;
+    };
+    std::vector<Piece> pieces;
+    size_t total = 0;
+    for (size_t k = 0; k < parts.size(); k++) {
+        // an index becomes five floats: smaller pieces
+        const size_t step = parts[k].dst ? kFetchSlot : kFetchSlot / 4;
+        for (size_t o = 0; o < parts[k].bytes; o += step) pieces.push_back({(int)k, o, std::min(step, parts[k].bytes - o)});
+        total += parts[k].bytes;
+    }
+    size_t want = std::min<size_t>({(size_t)std::max(1u, std::thread::hardware_concurrency()), (size_t)kFetchThreads, pieces.size(),
+                                    total / kFetchSlot + 1});
+    if (total <= kFetchSlot) want = 1;
+    for (size_t w = 0; w < want; w++) {
+        if (!c->fetch_slot[w]) TM_CUDA(c, cudaMallocHost((void**)&c->fetch_slot[w], kFetchSlot));
+        if (!c->fetch_stream[w]) TM_CUDA(c, cudaStreamCreateWithFlags(&c->fetch_stream[w], cudaStreamNonBlocking));
+    }
+    auto consume = [&](const Piece& p, const char* host) {
+        const FetchPart& f = parts[p.part];
+        if (f.dst) memcpy(f.dst + p.off, host, p.bytes);
+        else decode_best(c, reinterpret_cast<const int*>(host), p.bytes / sizeof(int), p.off / sizeof(int), to);
+    };
+    if (want == 1) {
+        // all pieces that fit the slot together, one wait for them
+        size_t k = 0;
+        while (k < pieces.size()) {
+            size_t used = 0, e = k;
+            for (; e < pieces.size() && used + pieces[e].bytes <= kFetchSlot; e++) {
+                TM_CUDA(c, cudaMemcpyAsync(c->fetch_slot[0] + used, (const char*)parts[pieces[e].part].src + pieces[e].off,
+                                           pieces[e].bytes, cudaMemcpyDeviceToHost, c->fetch_stream[0]));
+                used += pieces[e].bytes;
+            }
+            TM_CUDA(c, cudaStreamSynchronize(c->fetch_stream[0]));
+            used = 0;
+            for (; k < e; k++) {
+                consume(pieces[k], c->fetch_slot[0] + used);
+                used += pieces[k].bytes;
+            }
+        }
+        return TM_OK;
+    }
+    std::atomic<size_t> next{0};
+    std::atomic<int> failed{(int)cudaSuccess};
+    auto work = [&](int w) {
+        cudaError_t e = cudaSetDevice(c->device);
+        while (e == cudaSuccess && failed.load() == (int)cudaSuccess) {
+            const size_t k = next++;
+            if (k >= pieces.size()) break;
+            const Piece& p = pieces[k];
+            e = cudaMemcpyAsync(c->fetch_slot[w], (const char*)parts[p.part].src + p.off, p.bytes, cudaMemcpyDeviceToHost,
+                                c->fetch_stream[w]);
+            if (e == cudaSuccess) e = cudaStreamSynchronize(c->fetch_stream[w]);
+            if (e == cudaSuccess) consume(p, c->fetch_slot[w]);
+        }
+        if (e != cudaSuccess) failed = (int)e;
+    };
+    std::vector<std::thread> pool;
+    try {
+        pool.reserve(want);
+        for (size_t w = 1; w < want; w++) pool.emplace_back(work, (int)w);
+    } catch (...) {
+        // no more threads: those that started and this one do the work
+    }
+    work(0);
+    for (auto& th : pool) th.join();
+    if (failed != (int)cudaSuccess) return set_err(c, TM_ERR_CUDA, "result copy: %s", cudaGetErrorString((cudaError_t)failed.load()));
+    return TM_OK;
 }
 
 // The two used columns of RotationMatrix::SetToEulerRotation (matrix.cpp:490-510)
@@ -1349,67 +1475,17 @@ int tm_get_results(tm_ctx* c, float* mip, float* best_psi, float* best_theta, fl
     const size_t n = (size_t)c->X * c->Y;
     int rc = wait_stream(c, 3600.0);
     if (rc != TM_OK) return rc;
-    // the best-orientation map first: host threads decode it while this
-    // thread copies the other maps
-    std::vector<std::thread> pool;
-    const bool want_angles = best_psi || best_theta || best_phi || best_defocus || best_pixel_size;
-    if (want_angles) {
-        if (!c->best_host) TM_CUDA(c, cudaMallocHost((void**)&c->best_host, sizeof(int) * n));
-        TM_CUDA(c, cudaMemcpy(c->best_host, c->best, sizeof(int) * n, cudaMemcpyDeviceToHost));
-        const int* best = c->best_host;
-        // decode global orientation indices into angles and plane offsets, in parallel
-        auto decode = [c, best, best_psi, best_theta, best_phi, best_defocus, best_pixel_size](size_t i0, size_t i1) {
-            for (size_t i = i0; i < i1; i++) {
-                const int g = best[i];
-                float psi = 0, th = 0, ph = 0, df = 0, px = 0;
-                if (g >= 0) {
-                    // planes are few: linear scan from the back (most recent first)
-                    for (size_t k = c->planes.size(); k-- > 0;) {
-                        const Plane& p = c->planes[k];
-                        if (g >= p.base && g < p.base + p.n) {
-                            const float* ang = c->angle_lists[p.angles_id].data() + 3 * (size_t)(g - p.base);
-                            ph = ang[0];
-                            th = ang[1];
-                            psi = ang[2];
-                            df = p.defocus;
-                            px = p.pixel;
-                            break;
-                        }
-                    }
-                }
-                if (best_psi) best_psi[i] = psi;
-                if (best_theta) best_theta[i] = th;
-                if (best_phi) best_phi[i] = ph;
-                if (best_defocus) best_defocus[i] = df;
-                if (best_pixel_size) best_pixel_size[i] = px;
-            }
-        };
-        unsigned nt = std::thread::hardware_concurrency();
-        nt = nt < 1 ? 1 : (nt > 32 ? 32 : nt);
-        if (n < ((size_t)1 << 16)) nt = 1;
-        const size_t chunk = (n + nt - 1) / nt;
-        for (unsigned k = 0; k < nt; k++) {
-            const size_t i0 = k * chunk, i1 = std::min(n, i0 + chunk);
-            if (i0 < i1) pool.emplace_back(decode, i0, i1);
-        }
-    }
-    auto join = [&pool] {
-        for (auto& th : pool) th.join();
-        pool.clear();
-    };
-    cudaError_t e = cudaSuccess;
-    if (mip && e == cudaSuccess) e = cudaMemcpy(mip, c->mip, sizeof(float) * n, cudaMemcpyDeviceToHost);
-    if (sum && e == cudaSuccess) e = cudaMemcpy(sum, c->sum, sizeof(double) * n, cudaMemcpyDeviceToHost);
-    if (sum_of_squares && e == cudaSuccess)
-        e = cudaMemcpy(sum_of_squares, c->sumsq, sizeof(double) * n, cudaMemcpyDeviceToHost);
-    if (histogram && e == cudaSuccess) {
-        std::vector<unsigned long long> h(c->d.histogram_bins);
-        e = cudaMemcpy(h.data(), c->hist, sizeof(unsigned long long) * h.size(), cudaMemcpyDeviceToHost);
-        if (e == cudaSuccess)
-            for (size_t i = 0; i < h.size(); i++) histogram[i] = (long long)h[i];
-    }
-    join();
-    if (e != cudaSuccess) return set_err(c, TM_ERR_CUDA, "result copy: %s", cudaGetErrorString(e));
+    std::vector<FetchPart> parts;
+    const DecodeTo to{best_psi, best_theta, best_phi, best_defocus, best_pixel_size};
+    if (best_psi || best_theta || best_phi || best_defocus || best_pixel_size) parts.push_back({c->best, sizeof(int) * n, nullptr});
+    if (mip) parts.push_back({c->mip, sizeof(float) * n, (char*)mip});
+    if (sum) parts.push_back({c->sum, sizeof(double) * n, (char*)sum});
+    if (sum_of_squares) parts.push_back({c->sumsq, sizeof(double) * n, (char*)sum_of_squares});
+    std::vector<unsigned long long> h(histogram ? c->d.histogram_bins : 0);
+    if (histogram) parts.push_back({c->hist, sizeof(unsigned long long) * h.size(), (char*)h.data()});
+    rc = fetch_parts(c, parts, to);
+    if (rc != TM_OK) return rc;
+    for (size_t i = 0; i < h.size(); i++) histogram[i] = (long long)h[i];
     return TM_OK;
 }
 
@@ -1600,33 +1676,10 @@ int tm_get_image_results(tm_ctx* c, int image, float* mip, float* best_psi, floa
     if (rc != TM_OK) return rc;
     const size_t n = (size_t)c->X * c->Y;
     const tm_ctx::Slot& sl = c->slots[image];
-    if (mip) TM_CUDA(c, cudaMemcpy(mip, sl.mip, sizeof(float) * n, cudaMemcpyDeviceToHost));
-    if (best_psi || best_theta || best_phi) {
-        std::vector<int> best(n);
-        TM_CUDA(c, cudaMemcpy(best.data(), sl.best, sizeof(int) * n, cudaMemcpyDeviceToHost));
-        // planes are in increasing base order: binary search for the plane of each index
-        std::vector<long long> bases(c->planes.size());
-        for (size_t k = 0; k < bases.size(); k++) bases[k] = c->planes[k].base;
-        for (size_t i = 0; i < n; i++) {
-            const int g = best[i];
-            float psi = 0, th = 0, ph = 0;
-            const auto it = std::upper_bound(bases.begin(), bases.end(), (long long)g);
-            if (g >= 0 && it != bases.begin()) {
-                const Plane& p = c->planes[(size_t)(it - bases.begin()) - 1];
-                const long long o = g - p.base;
-                if (o >= 0 && o < p.n) {
-                    const float* e = c->angle_lists[p.angles_id].data() + 3 * o;
-                    ph = e[0];
-                    th = e[1];
-                    psi = e[2];
-                }
-            }
-            if (best_psi) best_psi[i] = psi;
-            if (best_theta) best_theta[i] = th;
-            if (best_phi) best_phi[i] = ph;
-        }
-    }
-    return TM_OK;
+    std::vector<FetchPart> parts;
+    if (best_psi || best_theta || best_phi) parts.push_back({sl.best, sizeof(int) * n, nullptr});
+    if (mip) parts.push_back({sl.mip, sizeof(float) * n, (char*)mip});
+    return fetch_parts(c, parts, DecodeTo{best_psi, best_theta, best_phi, nullptr, nullptr});
 }
 
 int tm_destroy(tm_ctx* c) {
