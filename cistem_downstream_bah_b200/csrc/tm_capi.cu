@@ -41,8 +41,11 @@ struct Plane {
 
 struct Variant;
 
+// Threads and slot bytes of fetch_parts.  Page-locking costs about 0.7 ms per MB on a context's
+// first results (24 MB took 17 ms in one allocation and 35 in twelve), so that a thread is used
+// per MB of results and has a small slot.
 constexpr int kFetchThreads = 12;
-constexpr size_t kFetchSlot = (size_t)2 << 20;   // bytes
+constexpr size_t kFetchSlot = (size_t)512 << 10;
 
 }  // namespace
 
@@ -65,8 +68,9 @@ struct tm_ctx {
     double *sum = nullptr, *sumsq = nullptr;
     unsigned long long* hist = nullptr;
     int* err_flag = nullptr;
-    // result maps on their way to the host (fetch_parts): a page-locked slot and a stream per thread
-    char* fetch_slot[kFetchThreads] = {};
+    // result maps on their way to the host (fetch_parts): page-locked slots and a stream per thread
+    char* fetch_slab = nullptr;
+    size_t fetch_slots = 0;
     cudaStream_t fetch_stream[kFetchThreads] = {};
     int precision = TM_PRECISION_FP32;
     tmk::GenPlan gen_px{}, gen_py{}, gen_ph{};   // radix plans of X, Y and X/2 (sizes without compiled kernels)
@@ -542,8 +546,7 @@ void free_all(tm_ctx* c) {
             if (p) cudaFree(p);
     }
     c->slots.clear();
-    for (char* p : c->fetch_slot)
-        if (p) cudaFreeHost(p);
+    if (c->fetch_slab) cudaFreeHost(c->fetch_slab);
     for (cudaStream_t s : c->fetch_stream)
         if (s) cudaStreamDestroy(s);
     if (c->stream) cudaStreamDestroy(c->stream);
@@ -593,69 +596,67 @@ void decode_best(const tm_ctx* c, const int* best, size_t n, size_t at, const De
 // through page-locked slots, each by a thread that then moves its piece into the caller's memory:
 // that memory is usually fresh, and its page faults, one thread's work in a plain cudaMemcpy,
 // are most of the time (4096 x 4096 results, 671 MB of maps: 80-95 ms with plain copies).
-// Little data stays on the calling thread, as starting threads costs more there (256 x 256: 1.8
-// ms with 16 threads).
+// Up to 2 MB are copied plainly by the calling thread: starting threads and page-locking cost
+// more there (256 x 256: 1.8 ms with 16 threads).
 struct FetchPart {
     const void* src;      // device
     size_t bytes;
     char* dst;            // null: best-orientation indices to decode
 };
 int fetch_parts(tm_ctx* c, const std::vector<FetchPart>& parts, const DecodeTo& to) {
+    size_t total = 0;
+    for (const FetchPart& f : parts) total += f.bytes;
+    if (total <= (size_t)2 << 20) {
+        for (const FetchPart& f : parts) {
+            if (f.dst) {
+                TM_CUDA(c, cudaMemcpy(f.dst, f.src, f.bytes, cudaMemcpyDeviceToHost));
+            } else {
+                std::vector<int> best(f.bytes / sizeof(int));
+                TM_CUDA(c, cudaMemcpy(best.data(), f.src, f.bytes, cudaMemcpyDeviceToHost));
+                decode_best(c, best.data(), best.size(), 0, to);
+            }
+        }
+        return TM_OK;
+    }
     struct Piece {
         int part;
         size_t off, bytes;
     };
     std::vector<Piece> pieces;
-    size_t total = 0;
     for (size_t k = 0; k < parts.size(); k++) {
         // an index becomes five floats: smaller pieces
         const size_t step = parts[k].dst ? kFetchSlot : kFetchSlot / 4;
         for (size_t o = 0; o < parts[k].bytes; o += step) pieces.push_back({(int)k, o, std::min(step, parts[k].bytes - o)});
-        total += parts[k].bytes;
     }
-    size_t want = std::min<size_t>({(size_t)std::max(1u, std::thread::hardware_concurrency()), (size_t)kFetchThreads, pieces.size(),
-                                    total / kFetchSlot + 1});
-    if (total <= kFetchSlot) want = 1;
-    for (size_t w = 0; w < want; w++) {
-        if (!c->fetch_slot[w]) TM_CUDA(c, cudaMallocHost((void**)&c->fetch_slot[w], kFetchSlot));
+    const size_t want = std::min<size_t>({(size_t)std::max(1u, std::thread::hardware_concurrency()), (size_t)kFetchThreads,
+                                          pieces.size(), total >> 20});
+    if (c->fetch_slots < want) {
+        if (c->fetch_slab) cudaFreeHost(c->fetch_slab);
+        c->fetch_slab = nullptr;
+        c->fetch_slots = 0;
+        TM_CUDA(c, cudaMallocHost((void**)&c->fetch_slab, want * kFetchSlot));
+        c->fetch_slots = want;
+    }
+    for (size_t w = 0; w < want; w++)
         if (!c->fetch_stream[w]) TM_CUDA(c, cudaStreamCreateWithFlags(&c->fetch_stream[w], cudaStreamNonBlocking));
-    }
     auto consume = [&](const Piece& p, const char* host) {
         const FetchPart& f = parts[p.part];
         if (f.dst) memcpy(f.dst + p.off, host, p.bytes);
         else decode_best(c, reinterpret_cast<const int*>(host), p.bytes / sizeof(int), p.off / sizeof(int), to);
     };
-    if (want == 1) {
-        // all pieces that fit the slot together, one wait for them
-        size_t k = 0;
-        while (k < pieces.size()) {
-            size_t used = 0, e = k;
-            for (; e < pieces.size() && used + pieces[e].bytes <= kFetchSlot; e++) {
-                TM_CUDA(c, cudaMemcpyAsync(c->fetch_slot[0] + used, (const char*)parts[pieces[e].part].src + pieces[e].off,
-                                           pieces[e].bytes, cudaMemcpyDeviceToHost, c->fetch_stream[0]));
-                used += pieces[e].bytes;
-            }
-            TM_CUDA(c, cudaStreamSynchronize(c->fetch_stream[0]));
-            used = 0;
-            for (; k < e; k++) {
-                consume(pieces[k], c->fetch_slot[0] + used);
-                used += pieces[k].bytes;
-            }
-        }
-        return TM_OK;
-    }
     std::atomic<size_t> next{0};
     std::atomic<int> failed{(int)cudaSuccess};
     auto work = [&](int w) {
+        char* const slot = c->fetch_slab + w * kFetchSlot;
         cudaError_t e = cudaSetDevice(c->device);
         while (e == cudaSuccess && failed.load() == (int)cudaSuccess) {
             const size_t k = next++;
             if (k >= pieces.size()) break;
             const Piece& p = pieces[k];
-            e = cudaMemcpyAsync(c->fetch_slot[w], (const char*)parts[p.part].src + p.off, p.bytes, cudaMemcpyDeviceToHost,
+            e = cudaMemcpyAsync(slot, (const char*)parts[p.part].src + p.off, p.bytes, cudaMemcpyDeviceToHost,
                                 c->fetch_stream[w]);
             if (e == cudaSuccess) e = cudaStreamSynchronize(c->fetch_stream[w]);
-            if (e == cudaSuccess) consume(p, c->fetch_slot[w]);
+            if (e == cudaSuccess) consume(p, slot);
         }
         if (e != cudaSuccess) failed = (int)e;
     };

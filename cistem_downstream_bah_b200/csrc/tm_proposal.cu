@@ -37,7 +37,17 @@ namespace tmp {
 
 constexpr int kC1 = 32, kC2 = 64, kC3 = 128, kC4 = 128, kOut = 4;
 constexpr int kThreads = 256;
-constexpr int kMaxGroups = 4;   // output-channel groups of a conv block (COB <= 32)
+
+// ----------------------------------------------------------------------------------------------
+// Two FP32 multiply-adds in one issue slot (sm_100's fma.f32x2, each half rounded as fmaf)
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+    float2 r;
+    asm("{\n\t.reg .b64 p, q, s, t;\n\tmov.b64 p, {%2, %3};\n\tmov.b64 q, {%4, %5};\n\tmov.b64 s, {%6, %7};\n\t"
+        "fma.rn.f32x2 t, p, q, s;\n\tmov.b64 {%0, %1}, t;\n\t}"
+        : "=f"(r.x), "=f"(r.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+    return r;
+}
 
 // ----------------------------------------------------------------------------------------------
 // 3x3 convolution, zero padding 1, NCHW.  out[n][o][y][x] = b[o] + sum_i sum_k
@@ -45,46 +55,57 @@ constexpr int kMaxGroups = 4;   // output-channel groups of a conv block (COB <=
 // kernel is the backward-data pass of a forward conv whose weights are
 // Wf[co][ci][3][3]: W(o, i, ky, kx) = Wf[i][o][2-ky][2-kx] (o runs over the
 // forward conv's input channels, i over its output channels), no bias, no ReLU.
+// Every output is one chain of multiply-adds over i, then ky, then kx.
 //
-// Block: a TH x TW tile of output pixels (TH = TW = min(16, H)) times COB output
-// channels (COB = 8 x groups, groups = min(256 / P, 4)); thread t < P x groups
-// computes pixel t % P for COT = 8 channels.  Input channels go through shared
-// memory CIB = 8 at a time with their halo.
-template <bool FLIP>
-__global__ void __launch_bounds__(kThreads)
+// Block: a TW x TW tile of output pixels times COB output channels; a thread computes
+// PXT pixels of a row x 8 channels, channels in pairs (two multiply-adds per
+// instruction, a pair's weights being adjacent in shared memory): 48 such instructions per
+// input channel and kernel row for 8 shared-memory loads.  (One pixel x 8 channels with
+// 9 loads per 8 multiply-adds: the shared-memory pipe bound it at a sixth of the FP32 rate, 200-417
+// us for the layers of 128 tiles of 64 x 64; 69-97 us now.)  Input channels go through
+// shared memory CIB at a time with their halo.
+template <int TW>
+struct ConvTile {
+    static constexpr int CIB = 8, COT = 8;
+    static constexpr int PXT = TW < 4 ? TW : 4;
+    static constexpr int PG = TW * TW / PXT;                            // pixel groups
+    static constexpr int CG = PG >= 64 ? 4 : PG >= 16 ? 8 : 16;         // channel groups
+    static constexpr int COB = CG * COT, NT = PG * CG;
+    static constexpr int PITCH = (TW + 2 + 3) / 4 * 4;                  // row pitch of the input tile, 16-byte aligned
+};
+
+template <bool FLIP, int TW>
+__global__ void __launch_bounds__(ConvTile<TW>::NT)
 k_conv3x3(const float* __restrict__ in, const __nv_bfloat16* __restrict__ w, const float* __restrict__ bias,
-          float* __restrict__ out, int Ci, int Co, int H, int W, int relu) {
-    constexpr int CIB = 8, COT = 8;
-    const int TH = H < 16 ? H : 16, TW = W < 16 ? W : 16;
-    const int P = TH * TW;
-    const int groups = kThreads / P < kMaxGroups ? kThreads / P : kMaxGroups;   // P divides 256
-    const int COB = groups * COT;
-    const int tiles_x = W / TW;
-    const int ty0 = (blockIdx.x / tiles_x) * TH, tx0 = (blockIdx.x % tiles_x) * TW;
+          float* __restrict__ out, int Ci, int Co, int H, int relu) {
+    using CT = ConvTile<TW>;
+    constexpr int CIB = CT::CIB, PXT = CT::PXT, COB = CT::COB, NT = CT::NT, PITCH = CT::PITCH, E = TW + 2;
+    __shared__ __align__(16) float s_in[CIB][E][PITCH];
+    __shared__ __align__(16) float s_w[CIB][9][COB];
+    const int tiles_x = H / TW;
+    const int ty0 = (blockIdx.x / tiles_x) * TW, tx0 = (blockIdx.x % tiles_x) * TW;
     const int co0 = blockIdx.y * COB;
     const int n = blockIdx.z;
     const int t = threadIdx.x;
-    const int pix = t % P, grp = t / P;
-    const int py = pix / TW, px = pix % TW;
-    __shared__ float s_in[CIB][18 * 18];
-    __shared__ float s_w[kMaxGroups * COT * CIB * 9];
-    const bool active = grp < groups;
-    float acc[COT];
+    const int pg = t % CT::PG, cg = t / CT::PG;
+    const int py = pg / (TW / PXT), px = pg % (TW / PXT) * PXT;
+    float2 acc[PXT][4];
 #pragma unroll
-    for (int j = 0; j < COT; j++) acc[j] = 0.0f;
-    const int HW = (TH + 2) * (TW + 2);
+    for (int p = 0; p < PXT; p++)
+#pragma unroll
+        for (int j = 0; j < 4; j++) acc[p][j] = make_float2(0.f, 0.f);
     for (int ci0 = 0; ci0 < Ci; ci0 += CIB) {
         // input tile with halo
-        for (int e = t; e < CIB * HW; e += kThreads) {
-            const int c = e / HW, r = e % HW;
-            const int yy = ty0 + r / (TW + 2) - 1, xx = tx0 + r % (TW + 2) - 1;
+        for (int e = t; e < CIB * E * E; e += NT) {
+            const int c = e / (E * E), r = e % (E * E);
+            const int yy = ty0 + r / E - 1, xx = tx0 + r % E - 1;
             const int ci = ci0 + c;
             float v = 0.0f;
-            if (ci < Ci && yy >= 0 && yy < H && xx >= 0 && xx < W) v = in[(((size_t)n * Ci + ci) * H + yy) * W + xx];
-            s_in[c][r] = v;
+            if (ci < Ci && yy >= 0 && yy < H && xx >= 0 && xx < H) v = in[(((size_t)n * Ci + ci) * H + yy) * H + xx];
+            s_in[c][r / E][r % E] = v;
         }
-        // weights of COB output channels x CIB input channels
-        for (int e = t; e < COB * CIB * 9; e += kThreads) {
+        // weights of COB output channels x CIB input channels, channel fastest
+        for (int e = t; e < COB * CIB * 9; e += NT) {
             const int o = e / (CIB * 9), r = e % (CIB * 9);
             const int c = r / 9, k = r % 9;
             const int co = co0 + o, ci = ci0 + c;
@@ -93,73 +114,185 @@ k_conv3x3(const float* __restrict__ in, const __nv_bfloat16* __restrict__ w, con
                 if (!FLIP) v = __bfloat162float(w[((size_t)co * Ci + ci) * 9 + k]);
                 else v = __bfloat162float(w[((size_t)ci * Co + co) * 9 + (8 - k)]);
             }
-            s_w[e] = v;
+            s_w[c][k][o] = v;
         }
         __syncthreads();
-        for (int c = 0; c < CIB && active; c++) {
+#pragma unroll 2
+        for (int c = 0; c < CIB; c++) {
 #pragma unroll
-            for (int k = 0; k < 9; k++) {
-                const float v = s_in[c][(py + k / 3) * (TW + 2) + px + k % 3];
+            for (int ky = 0; ky < 3; ky++) {
+                const float* row = &s_in[c][py + ky][px];
+                float v[PXT + 2];
+                if constexpr (PXT == 4) {
+                    const float4 a = *reinterpret_cast<const float4*>(row);
+                    const float2 b = *reinterpret_cast<const float2*>(row + 4);
+                    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y;
+                } else {
 #pragma unroll
-                for (int j = 0; j < COT; j++) acc[j] = fmaf(v, s_w[((grp * COT + j) * CIB + c) * 9 + k], acc[j]);
+                    for (int p = 0; p < PXT + 2; p++) v[p] = row[p];
+                }
+#pragma unroll
+                for (int kx = 0; kx < 3; kx++) {
+                    const float4* wp = reinterpret_cast<const float4*>(&s_w[c][ky * 3 + kx][cg * CT::COT]);
+                    const float4 w0 = wp[0], w1 = wp[1];
+                    const float2 wj[4] = {make_float2(w0.x, w0.y), make_float2(w0.z, w0.w), make_float2(w1.x, w1.y),
+                                          make_float2(w1.z, w1.w)};
+#pragma unroll
+                    for (int p = 0; p < PXT; p++)
+#pragma unroll
+                        for (int j = 0; j < 4; j++) acc[p][j] = fma2(make_float2(v[p + kx], v[p + kx]), wj[j], acc[p][j]);
+                }
             }
         }
         __syncthreads();
     }
-    if (!active) return;
     const int y = ty0 + py, x = tx0 + px;
 #pragma unroll
-    for (int j = 0; j < COT; j++) {
-        const int co = co0 + grp * COT + j;
+    for (int j = 0; j < CT::COT; j++) {
+        const int co = co0 + cg * CT::COT + j;
         if (co >= Co) continue;
-        float v = acc[j] + (bias ? bias[co] : 0.0f);
-        if (relu) v = fmaxf(v, 0.0f);
-        out[(((size_t)n * Co + co) * H + y) * W + x] = v;
+        const float b = bias ? bias[co] : 0.0f;
+#pragma unroll
+        for (int p = 0; p < PXT; p++) {
+            float v = (j & 1 ? acc[p][j / 2].y : acc[p][j / 2].x) + b;
+            if (relu) v = fmaxf(v, 0.0f);
+            out[(((size_t)n * Co + co) * H + y) * H + x + p] = v;
+        }
     }
 }
 
-// Weight and bias gradients of a 3x3 conv: dW[o][i][k] = sum_n sum_p g[n][o][p] *
-// in[n][i][p + k - (1,1)], db[o] = sum_n sum_p g[n][o][p].  One block per
-// (o, i) pair and image chunk; the nine sums are reduced in the block and added
-// to dW with atomics (dW and db are zeroed before the backward pass).
+// Weight and bias gradients of a 3x3 conv on W x W maps: dW[o][i][k] = sum_n sum_p g[n][o][p] *
+// in[n][i][p + k - (1,1)], db[o] = sum_n sum_p g[n][o][p].  A block takes 32 output x 8 input
+// channels and a share of the pixels, 256 at a time (a band of rows, or several whole maps)
+// through shared memory; a thread holds the nine sums of 4 output channels x 1
+// input channel over a quarter of them, output channels in pairs: 144 two-wide multiply-adds per 8
+// pixels of a row for 38 loads.  The quarters are added in the block, the blocks with
+// atomics (dW and db are zeroed before the backward pass).  (One block per channel pair read
+// every map from memory once per pair: 0.6-1.95 ms per layer of 128 tiles of 64 x 64; now
+// 0.1-0.2 ms.)
+template <int W>
+struct WGrad {
+    static constexpr int OB = 32, IB = 8, PX = 256;
+    static constexpr int RB = W * W <= PX ? W : PX / W;        // rows of a map per step
+    static constexpr int NI = PX / (RB * W);                   // maps per step
+    static constexpr int SL = W < 8 ? W : 8;                   // pixels of a row per inner step
+    static constexpr int GP = OB + 4;                          // pitch of a pixel's gradients
+    static constexpr int E = W + 2;
+    static constexpr int IN = NI * (RB + 2) * E * IB;
+    static constexpr int SMEM = (PX * GP + IN) * 4;
+    static_assert(IN >= 0 && SMEM >= 3 * 64 * 40 * 4, "the block reduction reuses the staging buffers");
+};
+
+template <int W>
 __global__ void __launch_bounds__(kThreads)
-k_conv3x3_wgrad(const float* __restrict__ in, const float* __restrict__ g, float* dW, float* db, int N, int Ci, int Co,
-                int H, int W, int n_chunk) {
-    const int o = blockIdx.x / Ci, i = blockIdx.x % Ci;
-    const int n0 = blockIdx.y * n_chunk, n1 = min(N, n0 + n_chunk);
-    const int HWp = H * W;
-    float s[10];
+k_conv3x3_wgrad(const float* __restrict__ in, const float* __restrict__ g, float* dW, float* db, int N, int Ci, int Co, int units) {
+    using WG = WGrad<W>;
+    constexpr int OB = WG::OB, IB = WG::IB, PX = WG::PX, RB = WG::RB, NI = WG::NI, SL = WG::SL, GP = WG::GP, E = WG::E;
+    extern __shared__ __align__(16) float wsm[];
+    float* const s_g = wsm;                 // [pixel][output channel]
+    float* const s_in = wsm + PX * GP;      // [map][row][column][input channel], with the halo
+    const int itiles = (Ci + IB - 1) / IB;
+    const int o0 = blockIdx.x / itiles * OB, i0 = blockIdx.x % itiles * IB;
+    const int t = threadIdx.x;
+    const int i = t & 7, og = (t >> 3) & 7, pq = t >> 6;   // input channel, group of 4 output channels, quarter
+    constexpr int bands = W / RB;
+    const int total = (N + NI - 1) / NI * bands;   // steps
+    float2 acc[2][9];
+    float2 accb[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
 #pragma unroll
-    for (int k = 0; k < 10; k++) s[k] = 0.0f;
-    // threads run over (image, pixel) pairs of the chunk, so that small maps keep them busy
-    const long long e1 = (long long)(n1 - n0) * HWp;
-    for (long long e = threadIdx.x; e < e1; e += kThreads) {
-        const int n = n0 + (int)(e / HWp), p = (int)(e % HWp);
-        const float gv = g[((size_t)n * Co + o) * HWp + p];
-        if (gv == 0.0f) continue;
-        const float* ip = in + ((size_t)n * Ci + i) * HWp;
-        const int y = p / W, x = p % W;
+    for (int h = 0; h < 2; h++)
 #pragma unroll
-        for (int k = 0; k < 9; k++) {
-            const int yy = y + k / 3 - 1, xx = x + k % 3 - 1;
-            if (yy >= 0 && yy < H && xx >= 0 && xx < W) s[k] = fmaf(gv, ip[yy * W + xx], s[k]);
+        for (int k = 0; k < 9; k++) acc[h][k] = make_float2(0.f, 0.f);
+    for (int u = blockIdx.y * units; u < min(total, (int)(blockIdx.y + 1) * units); u++) {
+        const int n0 = u / bands * NI, y0 = u % bands * RB;
+        bool unbounded = false;   // an input that is infinite or not a number
+        // gradients: 4 output channels of a pixel per thread and step
+        for (int e = t; e < PX * (OB / 4); e += kThreads) {
+            const int p = e % PX, o4 = e / PX * 4;
+            const int n = n0 + p / (RB * W), r = p % (RB * W);
+            float v[4] = {0.f, 0.f, 0.f, 0.f};
+            if (n < N) {
+                const float* gp = g + ((size_t)n * Co + o0 + o4) * (W * W) + y0 * W + r;
+#pragma unroll
+                for (int j = 0; j < 4; j++) v[j] = gp[(size_t)j * (W * W)];
+            }
+            *reinterpret_cast<float4*>(s_g + p * GP + o4) = make_float4(v[0], v[1], v[2], v[3]);
         }
-        s[9] += gv;
+        // inputs with the halo: 4 input channels of a pixel per thread and step
+        for (int e = t; e < NI * (RB + 2) * E * (IB / 4); e += kThreads) {
+            const int q = e % (NI * (RB + 2) * E), i4 = e / (NI * (RB + 2) * E) * 4;
+            const int n = n0 + q / ((RB + 2) * E), r = q % ((RB + 2) * E);
+            const int y = y0 + r / E - 1, x = r % E - 1;
+            float v[4] = {0.f, 0.f, 0.f, 0.f};
+            if (n < N && y >= 0 && y < W && x >= 0 && x < W) {
+                const float* ip = in + ((size_t)n * Ci + i0 + i4) * (W * W) + y * W + x;
+#pragma unroll
+                for (int j = 0; j < 4; j++)
+                    if (i0 + i4 + j < Ci) v[j] = ip[(size_t)j * (W * W)];
+#pragma unroll
+                for (int j = 0; j < 4; j++) unbounded = unbounded || !(fabsf(v[j]) <= FLT_MAX);
+            }
+            *reinterpret_cast<float4*>(s_in + q * IB + i4) = make_float4(v[0], v[1], v[2], v[3]);
+        }
+        // such an input counts only where its gradient is not zero (the ReLU masks it elsewhere)
+        const bool masked = __syncthreads_or(unbounded);
+        // this quarter's 64 pixels, SL of a row at a time
+#pragma unroll 1
+        for (int s0 = 64 * pq; s0 < 64 * pq + 64; s0 += SL) {
+            const int m = s0 / (RB * W), y = s0 / W % RB, x = s0 % W;
+            const float* ip = s_in + ((m * (RB + 2) + y) * E + x) * IB + i;
+            float v[3][SL + 2];
+#pragma unroll
+            for (int ky = 0; ky < 3; ky++)
+#pragma unroll
+                for (int p = 0; p < SL + 2; p++) v[ky][p] = ip[(ky * E + p) * IB];
+#pragma unroll
+            for (int p = 0; p < SL; p++) {
+                const float4 gv = *reinterpret_cast<const float4*>(s_g + (s0 + p) * GP + 4 * og);
+                const float2 ga = make_float2(gv.x, gv.y), gb = make_float2(gv.z, gv.w);
+                if (masked) {
+#pragma unroll
+                    for (int k = 0; k < 9; k++) {
+                        const float b = v[k / 3][p + k % 3];
+                        if (ga.x != 0.f) acc[0][k].x = fmaf(ga.x, b, acc[0][k].x);
+                        if (ga.y != 0.f) acc[0][k].y = fmaf(ga.y, b, acc[0][k].y);
+                        if (gb.x != 0.f) acc[1][k].x = fmaf(gb.x, b, acc[1][k].x);
+                        if (gb.y != 0.f) acc[1][k].y = fmaf(gb.y, b, acc[1][k].y);
+                    }
+                } else {
+#pragma unroll
+                    for (int k = 0; k < 9; k++) {
+                        const float2 b = make_float2(v[k / 3][p + k % 3], v[k / 3][p + k % 3]);
+                        acc[0][k] = fma2(ga, b, acc[0][k]);
+                        acc[1][k] = fma2(gb, b, acc[1][k]);
+                    }
+                }
+                accb[0].x += ga.x; accb[0].y += ga.y;
+                accb[1].x += gb.x; accb[1].y += gb.y;
+            }
+        }
+        __syncthreads();
     }
-    __shared__ float red[kThreads / 32][10];
+    // the quarters' sums: 40 values per (channel group, input channel)
+    float* const red = wsm;
+    auto value = [&](int e) -> float& {   // e = 10 j + k: output channel j, tap k (9: the bias)
+        const int j = e / 10, k = e % 10;
+        float2& a = k < 9 ? acc[j / 2][k] : accb[j / 2];
+        return j & 1 ? a.y : a.x;
+    };
+    if (pq > 0) {
 #pragma unroll
-    for (int k = 0; k < 10; k++) {
-        float v = s[k];
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
-        if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5][k] = v;
+        for (int e = 0; e < 40; e++) red[((pq - 1) * 40 + e) * 64 + (t & 63)] = value(e);
     }
     __syncthreads();
-    if (threadIdx.x < 10) {
-        float v = 0.0f;
-        for (int w8 = 0; w8 < kThreads / 32; w8++) v += red[w8][threadIdx.x];
-        if (threadIdx.x < 9) atomicAdd(&dW[((size_t)o * Ci + i) * 9 + threadIdx.x], v);
-        else if (i == 0) atomicAdd(&db[o], v);
+    if (pq == 0 && i0 + i < Ci) {
+#pragma unroll
+        for (int e = 0; e < 40; e++) {
+            const float v = value(e) + red[e * 64 + t] + red[(40 + e) * 64 + t] + red[(80 + e) * 64 + t];
+            const int o = o0 + 4 * og + e / 10, k = e % 10;
+            if (k < 9) atomicAdd(&dW[((size_t)o * Ci + i0 + i) * 9 + k], v);
+            else if (i0 + i == 0) atomicAdd(&db[o], v);
+        }
     }
 }
 
@@ -381,18 +514,27 @@ int grid_for(long long n) {
     return (int)(b < 148LL * 16 ? (b > 0 ? b : 1) : 148LL * 16);
 }
 
+template <bool FLIP, int TW>
+void conv_launch(tm_pnet* c, const float* in, const float* bias, float* out, const tmp::Layer& l, int n, int relu) {
+    using CT = tmp::ConvTile<TW>;
+    const int H = l.h, ci = FLIP ? l.co : l.ci, co = FLIP ? l.ci : l.co;
+    const dim3 grid((H / TW) * (H / TW), (co + CT::COB - 1) / CT::COB, n);
+    tmp::k_conv3x3<FLIP, TW><<<grid, CT::NT, 0, c->stream>>>(in, c->p16 + l.w, bias, out, ci, co, H, relu);
+}
+
 // launch of one conv: grid (spatial tiles, output-channel groups, images)
 int conv(tm_pnet* c, bool flip, const float* in, const float* bias, float* out, const tmp::Layer& l, int n, int relu) {
-    const int H = l.h;
-    const int TH = H < 16 ? H : 16;
-    const int P = TH * TH;
-    const int COB = (tmp::kThreads / P < tmp::kMaxGroups ? tmp::kThreads / P : tmp::kMaxGroups) * 8;
-    const int ci = flip ? l.co : l.ci, co = flip ? l.ci : l.co;
-    dim3 grid((H / TH) * (H / TH), (co + COB - 1) / COB, n);
-    if (flip)
-        tmp::k_conv3x3<true><<<grid, tmp::kThreads, 0, c->stream>>>(in, c->p16 + l.w, nullptr, out, ci, co, H, H, 0);
-    else
-        tmp::k_conv3x3<false><<<grid, tmp::kThreads, 0, c->stream>>>(in, c->p16 + l.w, bias, out, ci, co, H, H, relu);
+    if (flip) {
+        if (l.h >= 16) conv_launch<true, 16>(c, in, nullptr, out, l, n, 0);
+        else if (l.h == 8) conv_launch<true, 8>(c, in, nullptr, out, l, n, 0);
+        else if (l.h == 4) conv_launch<true, 4>(c, in, nullptr, out, l, n, 0);
+        else conv_launch<true, 2>(c, in, nullptr, out, l, n, 0);
+    } else {
+        if (l.h >= 16) conv_launch<false, 16>(c, in, bias, out, l, n, relu);
+        else if (l.h == 8) conv_launch<false, 8>(c, in, bias, out, l, n, relu);
+        else if (l.h == 4) conv_launch<false, 4>(c, in, bias, out, l, n, relu);
+        else conv_launch<false, 2>(c, in, bias, out, l, n, relu);
+    }
     PN_CUDA(c, cudaGetLastError());
     return TM_OK;
 }
@@ -414,17 +556,33 @@ int forward(tm_pnet* c, int n) {
     return TM_OK;
 }
 
-int wgrad(tm_pnet* c, const float* in, const float* g, const tmp::Layer& l, int n) {
-    const int pairs = l.ci * l.co;
-    int chunks = (148 * 8 + pairs - 1) / pairs;
-    if (chunks > n) chunks = n;
-    if (chunks < 1) chunks = 1;
-    const int n_chunk = (n + chunks - 1) / chunks;
-    dim3 grid(pairs, (n + n_chunk - 1) / n_chunk);
-    tmp::k_conv3x3_wgrad<<<grid, tmp::kThreads, 0, c->stream>>>(in, g, c->grad + l.w, c->grad + l.b, n, l.ci, l.co, l.h,
-                                                                l.h, n_chunk);
+template <int W>
+int wgrad_launch(tm_pnet* c, const float* in, const float* g, const tmp::Layer& l, int n) {
+    using WG = tmp::WGrad<W>;
+    if (WG::SMEM > 48 * 1024)
+        PN_CUDA(c, cudaFuncSetAttribute(tmp::k_conv3x3_wgrad<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, WG::SMEM));
+    // about four blocks per SM over the channel tiles and shares of the pixels
+    const int tiles = (l.co / WG::OB) * ((l.ci + WG::IB - 1) / WG::IB);
+    const int total = (n + WG::NI - 1) / WG::NI * (W / WG::RB);
+    int shares = (c->nsm * 4 + tiles - 1) / tiles;
+    if (shares > total) shares = total;
+    const int units = (total + shares - 1) / shares;
+    tmp::k_conv3x3_wgrad<W><<<dim3(tiles, (total + units - 1) / units), tmp::kThreads, WG::SMEM, c->stream>>>(
+        in, g, c->grad + l.w, c->grad + l.b, n, l.ci, l.co, units);
     PN_CUDA(c, cudaGetLastError());
     return TM_OK;
+}
+
+int wgrad(tm_pnet* c, const float* in, const float* g, const tmp::Layer& l, int n) {
+    switch (l.h) {
+        case 128: return wgrad_launch<128>(c, in, g, l, n);
+        case 64: return wgrad_launch<64>(c, in, g, l, n);
+        case 32: return wgrad_launch<32>(c, in, g, l, n);
+        case 16: return wgrad_launch<16>(c, in, g, l, n);
+        case 8: return wgrad_launch<8>(c, in, g, l, n);
+        case 4: return wgrad_launch<4>(c, in, g, l, n);
+        default: return wgrad_launch<2>(c, in, g, l, n);
+    }
 }
 
 // forward + loss + backward into c->grad; the loss sum into c->d_loss

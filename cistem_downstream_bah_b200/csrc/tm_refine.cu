@@ -501,9 +501,11 @@ int wait_refine(tm_refine_ctx* c, double limit_s) {
         cudaError_t e = cudaStreamQuery(c->stream);
         if (e == cudaSuccess) return TM_OK;
         if (e != cudaErrorNotReady) return rset_err(c, TM_ERR_CUDA, "device error: %s", cudaGetErrorString(e));
-        if (std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count() > limit_s)
-            return rset_err(c, TM_ERR_TIMEOUT, "stream did not finish within %.0f s", limit_s);
-        std::this_thread::sleep_for(std::chrono::microseconds(50));
+        const double el = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
+        if (el > limit_s) return rset_err(c, TM_ERR_TIMEOUT, "stream did not finish within %.0f s", limit_s);
+        // a batch of a few candidates takes tens of microseconds: yield for the first milliseconds
+        if (el < 2e-3) std::this_thread::yield();
+        else std::this_thread::sleep_for(std::chrono::microseconds(50));
     }
 }
 
