@@ -41,11 +41,13 @@ struct Plane {
 
 struct Variant;
 
-// Threads and slot bytes of fetch_parts.  Page-locking costs about 0.7 ms per MB on a context's
-// first results (24 MB took 17 ms in one allocation and 35 in twelve), so that a thread is used
-// per MB of results and has a small slot.
+// Most threads of fetch_parts.  Page-locking costs about 0.7 ms per MB on a context's first
+// results (24 MB: 17 ms in one allocation, 35 in twelve), while pieces below 2 MB cost
+// copies (4096 x 4096: 26 ms with 2 MB, 36 with 512 KB): the slots grow with the results.
 constexpr int kFetchThreads = 12;
-constexpr size_t kFetchSlot = (size_t)512 << 10;
+inline size_t fetch_slot_bytes(size_t total) {
+    return std::min<size_t>((size_t)2 << 20, std::max<size_t>((size_t)256 << 10, total / 192)) >> 16 << 16;
+}
 
 }  // namespace
 
@@ -70,7 +72,7 @@ struct tm_ctx {
     int* err_flag = nullptr;
     // result maps on their way to the host (fetch_parts): page-locked slots and a stream per thread
     char* fetch_slab = nullptr;
-    size_t fetch_slots = 0;
+    size_t fetch_bytes = 0;
     cudaStream_t fetch_stream[kFetchThreads] = {};
     int precision = TM_PRECISION_FP32;
     tmk::GenPlan gen_px{}, gen_py{}, gen_ph{};   // radix plans of X, Y and X/2 (sizes without compiled kernels)
@@ -623,19 +625,20 @@ int fetch_parts(tm_ctx* c, const std::vector<FetchPart>& parts, const DecodeTo& 
         size_t off, bytes;
     };
     std::vector<Piece> pieces;
+    const size_t slot_bytes = fetch_slot_bytes(total);
     for (size_t k = 0; k < parts.size(); k++) {
         // an index becomes five floats: smaller pieces
-        const size_t step = parts[k].dst ? kFetchSlot : kFetchSlot / 4;
+        const size_t step = parts[k].dst ? slot_bytes : slot_bytes / 4;
         for (size_t o = 0; o < parts[k].bytes; o += step) pieces.push_back({(int)k, o, std::min(step, parts[k].bytes - o)});
     }
     const size_t want = std::min<size_t>({(size_t)std::max(1u, std::thread::hardware_concurrency()), (size_t)kFetchThreads,
                                           pieces.size(), total >> 20});
-    if (c->fetch_slots < want) {
+    if (c->fetch_bytes < want * slot_bytes) {
         if (c->fetch_slab) cudaFreeHost(c->fetch_slab);
         c->fetch_slab = nullptr;
-        c->fetch_slots = 0;
-        TM_CUDA(c, cudaMallocHost((void**)&c->fetch_slab, want * kFetchSlot));
-        c->fetch_slots = want;
+        c->fetch_bytes = 0;
+        TM_CUDA(c, cudaMallocHost((void**)&c->fetch_slab, want * slot_bytes));
+        c->fetch_bytes = want * slot_bytes;
     }
     for (size_t w = 0; w < want; w++)
         if (!c->fetch_stream[w]) TM_CUDA(c, cudaStreamCreateWithFlags(&c->fetch_stream[w], cudaStreamNonBlocking));
@@ -647,7 +650,7 @@ int fetch_parts(tm_ctx* c, const std::vector<FetchPart>& parts, const DecodeTo& 
     std::atomic<size_t> next{0};
     std::atomic<int> failed{(int)cudaSuccess};
     auto work = [&](int w) {
-        char* const slot = c->fetch_slab + w * kFetchSlot;
+        char* const slot = c->fetch_slab + w * slot_bytes;
         cudaError_t e = cudaSetDevice(c->device);
         while (e == cudaSuccess && failed.load() == (int)cudaSuccess) {
             const size_t k = next++;

@@ -62,7 +62,7 @@ __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
 // instruction, a pair's weights being adjacent in shared memory): 48 such instructions per
 // input channel and kernel row for 8 shared-memory loads.  (One pixel x 8 channels with
 // 9 loads per 8 multiply-adds: the shared-memory pipe bound it at a sixth of the FP32 rate, 200-417
-// us for the layers of 128 tiles of 64 x 64; 69-97 us now.)  Input channels go through
+// us for the layers of 128 tiles of 64 x 64; 85-172 now.)  Input channels go through
 // shared memory CIB at a time with their halo.
 template <int TW>
 struct ConvTile {
