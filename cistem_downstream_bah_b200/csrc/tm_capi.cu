@@ -350,21 +350,20 @@ struct TcImpl {
 // template box T and the run-time-length passes of tm_generic.cuh.
 template <int T>
 struct GenImpl {
+    // two lines of X complex pairs in shared memory, else one line at a time
+    static bool pair_rows(int X) { return sizeof(float4) * 2 * X <= 232448; }
     static int configure(tm_ctx* c) {
-        TM_CUDA(c, cudaFuncSetAttribute(tmk::k_pass_a_gen<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)sizeof(float2) * 2 * c->X));
-        const int lw = tmk::gen_pass_b_lines(c->Y);
-        TM_CUDA(c, cudaFuncSetAttribute(lw == 4 ? tmk::k_pass_b_gen<4> : lw == 2 ? tmk::k_pass_b_gen<2> : tmk::k_pass_b_gen<1>,
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(float2) * 2 * lw * c->Y));
-        const int smem_c = (int)sizeof(float2) * (c->X % 2 ? 2 * c->X : c->X) + 4 * c->d.histogram_bins;
-        TM_CUDA(c, cudaFuncSetAttribute(pass_c_kernel(c->X), cudaFuncAttributeMaxDynamicSharedMemorySize, smem_c));
+        if (pair_rows(c->X))
+            TM_CUDA(c, cudaFuncSetAttribute(tmk::k_pass_a_gen2<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                            (int)sizeof(float4) * 2 * c->X));
+        else
+            TM_CUDA(c, cudaFuncSetAttribute(tmk::k_pass_a_gen<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                            (int)sizeof(float2) * 2 * c->X));
+        const tmk::GenColPass b = tmk::gen_col_pass(T, c->Y);
+        TM_CUDA(c, cudaFuncSetAttribute(b.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b.smem));
+        const tmk::GenRowPass r = tmk::gen_row_pass(c->X, c->XP, c->d.histogram_bins);
+        TM_CUDA(c, cudaFuncSetAttribute(r.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)r.smem));
         return TM_OK;
-    }
-    // the row pass for a width X: odd or even rows, 4, 8 or 16 pixels per thread
-    static auto pass_c_kernel(int X) -> void (*)(tmk::BatchArgs, int, int, tmk::GenPlan) {
-        const int mp = X <= 4 * tmk::kGenNT ? 4 : X <= 8 * tmk::kGenNT ? 8 : 16;
-        if (X % 2) return mp == 4 ? tmk::k_pass_c_gen<true, 4> : mp == 8 ? tmk::k_pass_c_gen<true, 8> : tmk::k_pass_c_gen<true, 16>;
-        return mp == 4 ? tmk::k_pass_c_gen<false, 4> : mp == 8 ? tmk::k_pass_c_gen<false, 8> : tmk::k_pass_c_gen<false, 16>;
     }
     static void prep(tm_ctx* c, tmk::BatchArgs& a, cudaStream_t s) {
         using SC = tmk::SliceCol<T>;
@@ -372,19 +371,18 @@ struct GenImpl {
         tmk::k_slice_colfft<T><<<dim3((T / 2 + 1 + SC::CB - 1) / SC::CB, a.nb), SC::NT, 0, s>>>(a);
         tmk::k_row_c2r<T><<<dim3(T / RC::ROWS, a.nb), RC::NT, 0, s>>>(a);
         tmk::k_norm<T><<<(a.nb + 7) / 8, 256, 0, s>>>(a, a.norm_pixels > 0 ? a.norm_pixels : (long long)c->X * c->Y);
-        tmk::k_pass_a_gen<T><<<dim3(T, a.nb), tmk::kGenNT, sizeof(float2) * 2 * c->X, s>>>(a, c->X, c->gen_px);
+        if (pair_rows(c->X)) tmk::k_pass_a_gen2<T><<<dim3(T / 2, a.nb), 256, sizeof(float4) * 2 * c->X, s>>>(a, c->X, c->gen_px);
+        else tmk::k_pass_a_gen<T><<<dim3(T, a.nb), tmk::kGenNT, sizeof(float2) * 2 * c->X, s>>>(a, c->X, c->gen_px);
     }
     static void pass_b(tm_ctx* c, tmk::BatchArgs& a, cudaStream_t s) {
         // the row pitch XP is a multiple of 4 columns (the variant's pass-B width)
-        const int lw = tmk::gen_pass_b_lines(c->Y);
-        const size_t smem = sizeof(float2) * 2 * lw * c->Y;
-        if (lw == 4) tmk::k_pass_b_gen<4><<<dim3(a.XP / 4, a.nb), tmk::kGenNT, smem, s>>>(a, T, c->Y, c->gen_py);
-        else if (lw == 2) tmk::k_pass_b_gen<2><<<dim3(a.XP / 2, a.nb), tmk::kGenNT, smem, s>>>(a, T, c->Y, c->gen_py);
-        else tmk::k_pass_b_gen<1><<<dim3(a.XP, a.nb), tmk::kGenNT, smem, s>>>(a, T, c->Y, c->gen_py);
+        const tmk::GenColPass b = tmk::gen_col_pass(T, c->Y);
+        const int ob = tmk::gen_col_orientations(b, a.XP, a.nb, c->nsm);
+        b.kernel<<<dim3(a.XP / b.columns, (a.nb + ob - 1) / ob), tmk::kGenNT, b.smem, s>>>(a, T, c->Y, ob, c->gen_py);
     }
     static void pass_c(tm_ctx* c, tmk::BatchArgs& a, cudaStream_t s) {
-        const size_t smem = sizeof(float2) * (c->X % 2 ? 2 * c->X : c->X) + 4 * a.hist_bins;
-        pass_c_kernel(c->X)<<<c->Y, tmk::kGenNT, smem, s>>>(a, c->X, c->Y, c->gen_ph);
+        const tmk::GenRowPass r = tmk::gen_row_pass(c->X, c->XP, a.hist_bins);
+        r.kernel<<<c->Y, r.threads, r.smem, s>>>(a, c->X, c->Y, c->gen_ph);
     }
     static int done(tm_ctx* c) {
         cudaError_t e = cudaGetLastError();
@@ -1531,10 +1529,8 @@ int tm_debug_stage_buffers(tm_ctx* c, const float* projection_filter, const floa
     if (projection) TM_CUDA(c, cudaMemcpy(projection, c->P, sizeof(float) * T * T, cudaMemcpyDeviceToHost));
     if (normalisation) TM_CUDA(c, cudaMemcpy(normalisation, c->norm, sizeof(float2), cudaMemcpyDeviceToHost));
     if (rows) TM_CUDA(c, cudaMemcpy2D(rows, hc * sizeof(float2), c->A, XP * sizeof(float2), hc * sizeof(float2), T, cudaMemcpyDeviceToHost));
-    if (columns && c->var->X == 0) {
-        TM_CUDA(c, cudaMemcpy2D(columns, hc * sizeof(float2), c->C, XP * sizeof(float2), hc * sizeof(float2), (size_t)c->Y, cudaMemcpyDeviceToHost));
-    } else if (columns) {
-        // out of the compiled geometries' tiles
+    if (columns) {
+        // out of C's tiles
         std::vector<float2> tiles((size_t)c->Y * XP);
         TM_CUDA(c, cudaMemcpy(tiles.data(), c->C, sizeof(float2) * tiles.size(), cudaMemcpyDeviceToHost));
         const size_t R = tmk::c_tile_rows(c->Y);

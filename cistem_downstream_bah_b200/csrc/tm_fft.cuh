@@ -489,9 +489,20 @@ __device__ __forceinline__ Pair pmul_conj(float2 ax, float2 ay, Pair b) {   // a
     const float2 y = cmul_conj(make_float2(ax.y, ay.y), make_float2(b.re.y, b.im.y));
     return {make_float2(x.x, y.x), make_float2(x.y, y.y)};
 }
-// a (c + i s) for a compile-time factor, two-wide, rounded as cmul
-__device__ __forceinline__ Pair pmulc(Pair a, float c, float s) {
-    return {fma2(a.re, both(c), mul2(a.im, both(-s))), fma2(a.re, both(s), mul2(a.im, both(c)))};
+// a (c + i s) for a compile-time factor, two-wide, rounded as cmul.  The factor's parts are
+// immediates inside the instruction block: as operands they are kept in register pairs over
+// the surrounding loops, and the kernels with many radices then spill them (the row pass at
+// 2700 pixels ran 115 M local loads beside 49 M shared ones).
+template <uint32_t C, uint32_t S, uint32_t NS>
+__device__ __forceinline__ Pair pmulc_bits(Pair a) {
+    Pair r;
+    asm("{\n\t.reg .b64 x, y, c, s, n, t, u;\n\tmov.b64 x, {%4, %5};\n\tmov.b64 y, {%6, %7};\n\t"
+        "mov.b64 c, {%8, %8};\n\tmov.b64 s, {%9, %9};\n\tmov.b64 n, {%10, %10};\n\t"
+        "mul.rn.f32x2 t, y, n;\n\tfma.rn.f32x2 t, x, c, t;\n\tmul.rn.f32x2 u, y, c;\n\tfma.rn.f32x2 u, x, s, u;\n\t"
+        "mov.b64 {%0, %1}, t;\n\tmov.b64 {%2, %3}, u;\n\t}"
+        : "=f"(r.re.x), "=f"(r.re.y), "=f"(r.im.x), "=f"(r.im.y)
+        : "f"(a.re.x), "f"(a.re.y), "f"(a.im.x), "f"(a.im.y), "n"(C), "n"(S), "n"(NS));
+    return r;
 }
 
 // ROT2: a2 still lacks a factor DIR i
@@ -524,6 +535,19 @@ __device__ __forceinline__ void pdft8(Pair* v) {
     v[7] = {fma2(t7.re, both(h), a3.re), fma2(t7.im, both(h), a3.im)};
 }
 
+// x W_R^K of both halves, as twc
+template <int R, int K, int DIR>
+__device__ __forceinline__ Pair ptwc(Pair x) {
+    constexpr int k = ((K % R) + R) % R;
+    if constexpr (k == 0) return x;
+    else {
+        static_assert(4 * k != R && 2 * k != R && 4 * k != 3 * R, "quarter turns are not needed here");
+        constexpr float c = (float)ct_cos(ct_angle(k, R));
+        constexpr float sn = (float)(DIR * ct_sin(ct_angle(k, R)));
+        return pmulc_bits<__builtin_bit_cast(uint32_t, c), __builtin_bit_cast(uint32_t, sn), __builtin_bit_cast(uint32_t, -sn)>(x);
+    }
+}
+
 // The 16-point DFT of both halves (rounded as dft16) as its two levels of four 4-point
 // transforms with the constants between, so that a caller can put loads, factors and stores
 // between the groups of four: level 1 takes x[r2], x[4 + r2], x[8 + r2], x[12 + r2], level 2 leaves
@@ -532,27 +556,94 @@ __device__ __forceinline__ void pdft8(Pair* v) {
 // v[10], is left to level 2 of q1 = 2 (pdft4's ROT2).
 template <int DIR>
 __device__ __forceinline__ void pdft16_mid(Pair* v) {
-    constexpr float c1 = 0.92387953251128675613f, s1 = 0.38268343236508977173f, h = 0.70710678118654752440f;
-    constexpr float sg = DIR < 0 ? -1.f : 1.f;
-    v[5] = pmulc(v[5], c1, sg * s1);
-    v[6] = pmulc(v[6], h, sg * h);
-    v[7] = pmulc(v[7], s1, sg * c1);
-    v[9] = pmulc(v[9], h, sg * h);
-    v[11] = pmulc(v[11], -h, sg * h);
-    v[13] = pmulc(v[13], s1, sg * c1);
-    v[14] = pmulc(v[14], -h, sg * h);
-    v[15] = pmulc(v[15], -c1, -sg * s1);
+    v[5] = ptwc<16, 1, DIR>(v[5]);
+    v[6] = ptwc<16, 2, DIR>(v[6]);
+    v[7] = ptwc<16, 3, DIR>(v[7]);
+    v[9] = ptwc<16, 2, DIR>(v[9]);
+    v[11] = ptwc<16, 6, DIR>(v[11]);
+    v[13] = ptwc<16, 3, DIR>(v[13]);
+    v[14] = ptwc<16, 6, DIR>(v[14]);
+    v[15] = ptwc<16, 9, DIR>(v[15]);
+}
+
+// dft3 of both halves (the factor h of its difference inside the last additions)
+template <int DIR>
+__device__ __forceinline__ void pdft3(Pair& a, Pair& b, Pair& c) {
+    constexpr float h = 0.86602540378443864676f, hd = DIR < 0 ? h : -h;
+    const Pair sm = padd(b, c), df = psub(b, c);
+    const Pair m = {fma2(both(-0.5f), sm.re, a.re), fma2(both(-0.5f), sm.im, a.im)};
+    a = padd(a, sm);
+    b = {fma2(both(hd), df.im, m.re), fma2(both(-hd), df.re, m.im)};
+    c = {fma2(both(-hd), df.im, m.re), fma2(both(hd), df.re, m.im)};
+}
+
+// dft9 of both halves, as dft_pq<3, 3>
+template <int DIR>
+__device__ __forceinline__ void pdft9(Pair* v) {
+    sfor<3>([&](auto rc) {
+        constexpr int r2 = decltype(rc)::value;
+        pdft3<DIR>(v[r2], v[3 + r2], v[6 + r2]);   // -> q1 at v[3 q1 + r2]
+        v[3 + r2] = ptwc<9, r2, DIR>(v[3 + r2]);
+        v[6 + r2] = ptwc<9, 2 * r2, DIR>(v[6 + r2]);
+    });
+    Pair o[9];
+#pragma unroll
+    for (int q1 = 0; q1 < 3; q1++) {
+        pdft3<DIR>(v[3 * q1], v[3 * q1 + 1], v[3 * q1 + 2]);
+#pragma unroll
+        for (int q2 = 0; q2 < 3; q2++) o[q1 + 3 * q2] = v[3 * q1 + q2];
+    }
+#pragma unroll
+    for (int i = 0; i < 9; i++) v[i] = o[i];
+}
+
+// R-point DFT of prime length as R^2 multiplications by compile-time constants
+template <int R, int DIR>
+__device__ __forceinline__ void pdft_prime(Pair* v) {
+    Pair o[R];
+    sfor<R>([&](auto kc) {
+        constexpr int k = decltype(kc)::value;
+        Pair acc = v[0];
+        sfor<R - 1>([&](auto ic) {
+            constexpr int i = decltype(ic)::value + 1;
+            acc = padd(acc, ptwc<R, (i * k) % R, DIR>(v[i]));
+        });
+        o[k] = acc;
+    });
+#pragma unroll
+    for (int i = 0; i < R; i++) v[i] = o[i];
+}
+
+template <int DIR>
+__device__ __forceinline__ void pdft16(Pair* v) {
+#pragma unroll
+    for (int g = 0; g < 4; g++) pdft4<DIR>(v[g], v[4 + g], v[8 + g], v[12 + g]);
+    pdft16_mid<DIR>(v);
+    Pair o[16];
+    sfor<4>([&](auto gc) {
+        constexpr int g = decltype(gc)::value;
+        pdft4<DIR, g == 2>(v[4 * g], v[4 * g + 1], v[4 * g + 2], v[4 * g + 3]);
+#pragma unroll
+        for (int k = 0; k < 4; k++) o[g + 4 * k] = v[4 * g + k];
+    });
+#pragma unroll
+    for (int i = 0; i < 16; i++) v[i] = o[i];
 }
 
 template <int RS, int DIR>
 __device__ __forceinline__ void pdft(Pair* v) {
-    if constexpr (RS == 8) pdft8<DIR>(v);
+    if constexpr (RS == 16) pdft16<DIR>(v);
+    else if constexpr (RS == 8) pdft8<DIR>(v);
     else if constexpr (RS == 4) pdft4<DIR>(v[0], v[1], v[2], v[3]);
-    else {
-        static_assert(RS == 2, "unsupported radix");
+    else if constexpr (RS == 9) pdft9<DIR>(v);
+    else if constexpr (RS == 3) pdft3<DIR>(v[0], v[1], v[2]);
+    else if constexpr (RS == 2) {
         const Pair a = v[0], b = v[1];
         v[0] = padd(a, b);
         v[1] = psub(a, b);
+    } else {
+        static_assert(RS == 5 || RS == 7 || RS == 11 || RS == 13, "unsupported radix");
+        pdft_prime<RS, DIR>(v);
     }
 }
 

@@ -65,11 +65,15 @@ __host__ __device__ constexpr int col_radix(int Y) { return Y % 3 == 0 ? 18 : 16
 // row pass gathers a row's 32-byte pieces by tensor-map copies; the blocks on the R rows
 // of a tile read it at about the same time, through the L2 (4.8-5.5 TB/s in a load-only
 // kernel, against 7.2 for whole rows; it needs 2.8).
-__host__ __device__ constexpr int c_tile_rows(int Y) { return Y % 8 == 0 ? 8 : 4; }
+__host__ __device__ constexpr int c_tile_rows(int Y) { return Y % 8 == 0 ? 8 : Y % 4 == 0 ? 4 : Y % 2 == 0 ? 2 : 1; }
+__host__ __device__ inline size_t c_index_rt(int Y, int o, int y, int kx, int XP) {
+    const int R = c_tile_rows(Y);
+    return (((size_t)o * (Y / R) + y / R) * (XP / 4) + kx / 4) * (4 * R) + (y % R) * 4 + kx % 4;
+}
 template <int Y>
 __host__ __device__ constexpr size_t c_index(int o, int y, int kx, int XP) {
     constexpr int R = c_tile_rows(Y);
-    static_assert(Y % R == 0, "heights are whole tiles");
+    static_assert(R >= 4, "compiled heights are whole tiles of at least 4 rows");
     return (((size_t)o * (Y / R) + y / R) * (XP / 4) + kx / 4) * (4 * R) + (y % R) * 4 + kx % 4;
 }
 // A row of C in the row pass's shared memory: its XP / 4 column groups arrive in c_row_boxes(XP)
