@@ -540,8 +540,11 @@ template <int R, int K, int DIR>
 __device__ __forceinline__ Pair ptwc(Pair x) {
     constexpr int k = ((K % R) + R) % R;
     if constexpr (k == 0) return x;
-    else {
-        static_assert(4 * k != R && 2 * k != R && 4 * k != 3 * R, "quarter turns are not needed here");
+    else if constexpr (2 * k == R) return {make_float2(-x.re.x, -x.re.y), make_float2(-x.im.x, -x.im.y)};
+    else if constexpr (4 * k == R || 4 * k == 3 * R) {
+        constexpr bool plus = (4 * k == R) == (DIR > 0);   // times +i, else -i
+        return plus ? Pair{make_float2(-x.im.x, -x.im.y), x.re} : Pair{x.im, make_float2(-x.re.x, -x.re.y)};
+    } else {
         constexpr float c = (float)ct_cos(ct_angle(k, R));
         constexpr float sn = (float)(DIR * ct_sin(ct_angle(k, R)));
         return pmulc_bits<__builtin_bit_cast(uint32_t, c), __builtin_bit_cast(uint32_t, sn), __builtin_bit_cast(uint32_t, -sn)>(x);
@@ -597,6 +600,36 @@ __device__ __forceinline__ void pdft9(Pair* v) {
     for (int i = 0; i < 9; i++) v[i] = o[i];
 }
 
+template <int RS, int DIR>
+__device__ __forceinline__ void pdft(Pair* v);
+
+// dft_pq of both halves
+template <int R1, int R2, int DIR>
+__device__ __forceinline__ void pdft_pq(Pair* v) {
+    constexpr int R = R1 * R2;
+    Pair u[R];
+    sfor<R2>([&](auto r2c) {
+        constexpr int r2 = decltype(r2c)::value;
+        Pair t[R1];
+#pragma unroll
+        for (int r1 = 0; r1 < R1; r1++) t[r1] = v[R2 * r1 + r2];
+        pdft<R1, DIR>(t);
+        sfor<R1>([&](auto q1c) {
+            constexpr int q1 = decltype(q1c)::value;
+            u[r2 * R1 + q1] = ptwc<R, r2 * q1, DIR>(t[q1]);
+        });
+    });
+#pragma unroll
+    for (int q1 = 0; q1 < R1; q1++) {
+        Pair t[R2];
+#pragma unroll
+        for (int r2 = 0; r2 < R2; r2++) t[r2] = u[r2 * R1 + q1];
+        pdft<R2, DIR>(t);
+#pragma unroll
+        for (int q2 = 0; q2 < R2; q2++) v[q1 + R1 * q2] = t[q2];
+    }
+}
+
 // R-point DFT of prime length as R^2 multiplications by compile-time constants
 template <int R, int DIR>
 __device__ __forceinline__ void pdft_prime(Pair* v) {
@@ -641,10 +674,122 @@ __device__ __forceinline__ void pdft(Pair* v) {
         const Pair a = v[0], b = v[1];
         v[0] = padd(a, b);
         v[1] = psub(a, b);
-    } else {
+    } else if constexpr (RS == 6) pdft_pq<3, 2, DIR>(v);
+    else if constexpr (RS == 12) pdft_pq<4, 3, DIR>(v);
+    else if constexpr (RS == 18) pdft_pq<9, 2, DIR>(v);
+    else {
         static_assert(RS == 5 || RS == 7 || RS == 11 || RS == 13, "unsupported radix");
         pdft_prime<RS, DIR>(v);
     }
+}
+
+// apply_twiddles on both halves, which share the powers of w
+template <int RS>
+__device__ __forceinline__ void papply_twiddles(Pair* e, float2 w) {
+    if constexpr (RS != 2 && RS != 4 && RS != 8 && RS != 16) {
+        float2 p[RS];
+        p[1] = w;
+#pragma unroll
+        for (int k = 2; k < RS; k++) p[k] = cmul(p[k >> 1], p[k - (k >> 1)]);
+#pragma unroll
+        for (int k = 1; k < RS; k++) e[k] = pmul(e[k], p[k]);
+    } else {
+        float2 p[RS];   // the powers of apply_twiddles: w^k = w^h w^(k - h), h the largest power of 2 below k
+        p[1] = w;
+#pragma unroll
+        for (int k = 2; k < RS; k++) {
+            const int h = k > 8 ? 8 : k > 4 ? 4 : k > 2 ? 2 : 1;
+            p[k] = k > 12 ? cmul(p[12], p[k - 12]) : cmul(p[h], p[k - h]);
+        }
+#pragma unroll
+        for (int k = 1; k < RS; k++) e[k] = pmul(e[k], p[k]);
+    }
+}
+
+// The base twiddles of a plan's stages in one array: stage s (from 1) takes Ns entries, entry k being
+// W_L^(k L / (Ns RS)), so that neighbouring threads read neighbouring entries.
+template <int L, int R>
+__host__ __device__ constexpr int stage_table_len(int s = Plan<L, R>::stages) {
+    int n = 0;
+    for (int i = 1; i < s; i++) n += Plan<L, R>::ns(i);
+    return n;
+}
+template <int L, int R>
+__device__ __forceinline__ void fill_stage_table(float2* dst, const Twiddles& tw, int tid, int nthreads) {
+    using PL = Plan<L, R>;
+    sfor<PL::stages>([&](auto sc) {
+        constexpr int s = decltype(sc)::value;
+        if constexpr (s > 0) {
+            constexpr int Ns = PL::ns(s);
+            for (int k = tid; k < Ns; k += nthreads) dst[stage_table_len<L, R>(s) + k] = tw.template w<-1>(k * (L / (Ns * PL::radix(s))), L);
+        }
+    });
+}
+
+// Place of element i with one spare element per D (0: none).  An address (t + P r or idxD + r Ns) is a
+// base plus a compile-time offset per r where no multiple of D falls inside a step.
+template <int D>
+__host__ __device__ constexpr int pad_at(int i) { return D ? i + i / (D ? D : 1) : i; }
+
+// fft on both halves.  Element i of a pair is buf[pad_at<D>(i) * WP]: WP pairs side by side, 16
+// bytes each, so that 8 lanes (WP pairs of 8 / WP neighbouring t) access 128 different bytes.
+// tab: the plan's stage table in shared memory.  act: this thread's outputs are wanted in buf
+// (padding lanes of a block pass false).
+template <int L, int R, int DIR, int WP, int D, bool FIRST_SYNC = true, class Sync>
+__device__ __forceinline__ void pfft(Pair (&v)[R], int t, float4* buf, const float2* tab, bool act, Sync sync) {
+    using PL = Plan<L, R>;
+    constexpr int P = PL::P;
+    sfor<PL::stages>([&](auto sc) {
+        constexpr int s = decltype(sc)::value;
+        constexpr int RS = PL::radix(s);
+        constexpr int Ns = PL::ns(s);
+        constexpr bool last = (s == PL::stages - 1);
+        if constexpr (s > 0) {
+            sync();
+            auto get = [&](Pair& p, const float4* at) {
+                const float4 f = *at;
+                p = {make_float2(f.x, f.y), make_float2(f.z, f.w)};
+            };
+            if constexpr (D == 0 || P % (D ? D : 1) == 0 || D % P == 0) {
+                const float4* rb = buf + pad_at<D % P == 0 && P < D ? 0 : D>(t) * WP;   // (t below P below D: no spare element)
+#pragma unroll
+                for (int r = 0; r < R; r++) get(v[r], rb + pad_at<D>(P * r) * WP);
+            } else {
+#pragma unroll
+                for (int r = 0; r < R; r++) get(v[r], buf + pad_at<D>(t + P * r) * WP);
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < R / RS; u++) {
+            const int b = t + P * u;
+            Pair e[RS];
+#pragma unroll
+            for (int r = 0; r < RS; r++) e[r] = v[u + r * (R / RS)];
+            if constexpr (s > 0) {
+                const float2 w = tab[stage_table_len<L, R>(s) + (last ? b : b % Ns)];   // b < L / RS, which is the last Ns
+                papply_twiddles<RS>(e, DIR < 0 ? w : conjf2(w));
+            }
+            pdft<RS, DIR>(e);
+            if constexpr (last) {
+#pragma unroll
+                for (int r = 0; r < RS; r++) v[u + r * (R / RS)] = e[r];
+            } else {
+                if (u == 0 && (FIRST_SYNC || s > 0)) sync();  // previous readers of buf are done
+                auto put = [](float4* at, Pair p) { *at = make_float4(p.re.x, p.re.y, p.im.x, p.im.y); };
+                if (act) {
+                    const int idxD = (b / Ns) * Ns * RS + (b % Ns);
+                    if constexpr (D == 0 || Ns % (D ? D : 1) == 0 || (Ns == 1 && D % RS == 0)) {
+                        float4* wb = buf + pad_at<D>(idxD) * WP;
+#pragma unroll
+                        for (int r = 0; r < RS; r++) put(wb + pad_at<D>(r * Ns) * WP, e[r]);
+                    } else {
+#pragma unroll
+                        for (int r = 0; r < RS; r++) put(buf + pad_at<D>(idxD + r * Ns) * WP, e[r]);
+                    }
+                }
+            }
+        }
+    });
 }
 
 }  // namespace tmfft

@@ -393,30 +393,32 @@ k_pass_a(BatchArgs a) {
 // Work items of the column passes: (column group, orientation).  A block owns
 // whole column groups, every orientation of a group in turn (its micrograph
 // values stay in TMEM), and the blocks take adjacent groups in rounds: block b
-// has groups b, b + nblk, b + 2 nblk, ...  All blocks then write rows of the
-// same orientation at about the same time, into adjacent 32-byte sectors of
-// each row, which the L2 merges into whole lines before writing them back.
-// (With each block on a contiguous run of items, the blocks wrote rows of
-// unrelated orientations one sector at a time, and the 4096 x 4096 column pass
-// took 2.3 times as long as with its stores going to L2-resident addresses.)
-// Groups left over after the whole rounds are split by orientation ranges over
-// the blocks that would otherwise idle.
+// has groups b, b + nblk, b + 2 nblk, ...  All blocks then read the same rows of A and of I',
+// 32 bytes of each, and write adjacent tiles at about the same time, so that the memory
+// sees whole lines.
+// Groups left over after the whole rounds are split by orientation ranges, each block
+// on one group, or, where that makes the longest block's list shorter, their items are shared out evenly, in
+// runs of consecutive orientations that can cross from one group to the next (257
+// groups on 148 blocks, 33 orientations: 0.60 -> 0.53 ms, 39 blocks idled in the last round; 132 groups on 592 blocks,
+// 96 orientations: 0.186 -> 0.175).
 struct ColSchedule {
-    int nb, nblk, b, rounds, tail_g, o_lo, n;
+    int nb, nblk, b, rounds, tail, n;   // tail: this block's first item of the groups left over
     __host__ __device__ ColSchedule(int ngroups, int nbatch, int blk, int nblocks) : nb(nbatch), nblk(nblocks), b(blk) {
         rounds = ngroups / nblk;
         const int rem = ngroups % nblk;
         const int parts = rem ? min(nb, nblk / rem) : 1;
-        int o_hi = 0;
-        tail_g = -1;
-        o_lo = 0;
-        if (rem && b < rem * parts) {
+        const int left = rem * nb, each = left / nblk, more = left - each * nblk;
+        int end = 0;
+        tail = 0;
+        if ((nb + parts - 1) / parts > each + (more > 0)) {
+            tail = b * each + min(b, more);
+            end = tail + each + (b < more);
+        } else if (b < rem * parts) {
             const int p = b / rem;
-            tail_g = rounds * nblk + b % rem;
-            o_lo = p * nb / parts;
-            o_hi = (p + 1) * nb / parts;
+            tail = b % rem * nb + p * nb / parts;
+            end = b % rem * nb + (p + 1) * nb / parts;
         }
-        n = rounds * nb + (o_hi - o_lo);
+        n = rounds * nb + end - tail;
     }
     // most items a block gets
     __host__ __device__ static int max_items(int ngroups, int nbatch, int nblocks) {
@@ -425,141 +427,121 @@ struct ColSchedule {
     // (group, orientation) of the block's idx-th item.  k_pass_b keeps the schedule
     // in shared memory (its fields cost no registers across the item loop);
     // k_pass_b_rg expands it into a list of items there.
-    __host__ __device__ void locate(int idx, int& g, int& o) const {
+    __host__ __device__ void locate(int idx, int& g, int& o) const { place(nb, nblk, b, rounds, tail, idx, g, o); }
+    // the same from the block's shared-memory copy, read afresh on every call
+    __device__ static void locate(const volatile ColSchedule* s, int idx, int& g, int& o) {
+        place(s->nb, s->nblk, s->b, s->rounds, s->tail, idx, g, o);
+    }
+
+private:
+    __host__ __device__ static void place(int nb, int nblk, int b, int rounds, int tail, int idx, int& g, int& o) {
         if (idx < rounds * nb) {
             g = (idx / nb) * nblk + b;
             o = idx % nb;
         } else {
-            g = tail_g;
-            o = o_lo + idx - rounds * nb;
-        }
-    }
-    // the same from the block's shared-memory copy, read afresh on every call
-    __device__ static void locate(const volatile ColSchedule* s, int idx, int& g, int& o) {
-        const int nb = s->nb, rounds = s->rounds;
-        if (idx < rounds * nb) {
-            g = (idx / nb) * s->nblk + s->b;
-            o = idx % nb;
-        } else {
-            g = s->tail_g;
-            o = s->o_lo + idx - rounds * nb;
+            const int i = tail + idx - rounds * nb;
+            g = rounds * nblk + i / nb;
+            o = i % nb;
         }
     }
 };
 static_assert(sizeof(ColSchedule) <= 48, "the schedule sits in the last 48 bytes of a column pass's shared memory");
 
 // --------------------------------------------------------------------------------------
-// k_pass_b: persistent; block = W columns x P threads (thread = c + W*j,
-// P = Y/V); work item = (group of G column chunks, orientation), orientation
-// fastest.  With 2-column chunks (tall micrographs, where 4 columns would need
-// more than 1024 threads) an item covers two chunks one after the other and
-// writes its 4 columns from shared memory, so every store fills whole 32-byte
-// row sectors (16-byte partial-sector stores cost DRAM read-modify-writes).
-// Each thread parks the V values of the prepared micrograph spectrum I' it
-// multiplies with in tensor memory (TMEM, 2V columns of its lane) for all
-// orientations of the chunk, which leaves shared memory to full complex
-// exchange buffers; a trailing partial warp (when W*P is not a multiple of 32)
-// reads its I' values from global memory instead, since tcgen05 loads are
-// whole-warp operations.  The rows of A for the next item stream in with
-// cp.async while the current item is transformed.  The forward transform
-// along y is pruned: MY = Y/L twiddled L-point transforms of the T rows of A
-// zero-padded to L (L = T for power-of-two heights).
+// k_pass_b: persistent; block = W columns x P / 2 threads (thread = cp + W/2 j, P = Y/V),
+// two adjacent columns per thread (tmfft::Pair); work item = (group of W columns,
+// orientation), orientation fastest.  Each thread parks the V values of the prepared
+// micrograph spectrum I' of its two columns in tensor memory (TMEM, 4V columns of its lane)
+// for all orientations of the group, which leaves shared memory to the exchange buffer, 16
+// bytes per element and column pair.  Blocks are padded to whole warps (tcgen05 loads
+// are whole-warp operations); the padding lanes repeat the last thread's work without storing it.
+// The rows of A for the next item stream in with cp.async while the current item is
+// transformed.  Twiddles come from tables of the stages' bases in shared memory (from the
+// L2, all warps of a block waited for them at each stage).
+// What bounds it: the FP32 pipe (44 % busy at 256 x 3888; one item's loads, butterflies and stores take turns
+// at the block's barriers), then its writes of C.  One column per thread -> this, 32
+// orientations of 4096 columns: 256 x 3888 1.52 -> 1.46 ms, 384 x 5832 3.36 -> 2.39; 33 of 2048 columns: 256 x 2916 0.70
+// -> 0.53, 256 x 2592 0.85 -> 0.70; 96 of 1024: 64 x 1024 0.21 -> 0.17; 96 of 512: 256 x 512 0.073 -> 0.059; below 0.02 ms
+// (32 x 256) a launch gains nothing.  (At 5832, both pairs of a thread one after the other, without spills but
+// with 11 warps: 2.73 ms.)
+// The forward transform along y is pruned: MY = Y/L twiddled L-point transforms
+// of the T rows of A zero-padded to L (L = T for power-of-two heights).
 template <int T, int Y>
 struct PassB {
-    // values per thread: the column radix.  (32 values -- two radix-16
-    // butterflies per thread and stage, 512 threads -- compiles and passes the
-    // same tests but measured no faster on 4096 x 4096.)
-    static constexpr int V = col_radix(Y);
-    static constexpr int P = Y / V;                                 // threads per column
-    // columns per block; 32 values per thread need 128 registers: 512 threads
-    static constexpr int W = V == 32 ? 4 : (16 * P <= 1024) ? 16 : (8 * P <= 1024) ? 8 : (4 * P <= 1024) ? 4 : 2;
-    static constexpr int NT = W * P;                                // threads per block
+    static constexpr int V = col_radix(Y);                          // values per thread: the column radix
+    static constexpr int P = Y / V;                                 // threads per column pair
+    static constexpr int W = P <= 16 ? 8 : 4;                       // columns per item: one tile of C, or two (at least two warps)
+    static constexpr int WP = W / 2;
+    static constexpr int NA = WP * P;                               // threads with columns of their own
+    static constexpr int NT = (NA + 31) / 32 * 32;
     static constexpr int L = prune_len(T, Y, V);                    // pruned forward length
     static constexpr int MY = Y / L, PT = L / V;
-    static constexpr int FULL_WARPS = NT / 32;
-    // chunks written back to back for one orientation, so that together they
-    // cover whole 32-byte sectors of a row (G > 1 only for 2-column chunks)
-    static constexpr int G = W >= 4 ? 1 : 4 / W;
-    static constexpr int WG = W * G;                                // columns per work item
-    // A 1024-thread block of at least 8 columns runs as NH = 2 independent
-    // halves of 512 threads (W/2 columns each, own named barrier), so that one
-    // half's transforms issue while the other waits at a barrier.  A warp then
-    // covers W/2 >= 4 adjacent columns, whole 32-byte sectors of each row.  (With
-    // 4 columns each half would write 16-byte halves of the sectors; measured at
-    // 4096 x 4096, the L2 did not merge them and the DRAM traffic of the pass
-    // rose from 11 to 30 GB per 128 orientations, so 4-column blocks stay whole.)
-    static constexpr int NH = (NT == 1024 && G == 1 && W >= 8) ? 2 : 1;
-    static constexpr int WL = W / NH;                               // columns interleaved in a warp
-    static constexpr int NTH = NT / NH;                             // threads per half
-    // bank skews (float2 units, half-warp = 16 lanes = (16/WL) values of j x WL columns)
-    static constexpr int RST = (tmfft::padded_len(L) + 15) / 16 * 16 + 1;       // == 1 (mod 16)
-    static constexpr int CS0 = (MY * RST > tmfft::padded_len(Y)) ? MY * RST : tmfft::padded_len(Y);
-    static constexpr int CS = (CS0 + 15) / 16 * 16 + 16 / WL;                 // == 16/WL (mod 16)
-    static constexpr size_t EXCH = (sizeof(float2) * WG * CS + 15) / 16 * 16;
-    static constexpr size_t ASZ = sizeof(float2) * T * WG;          // one A staging buffer
-    static constexpr int ABUFS = (EXCH + 2 * ASZ + 64 <= 232448) ? 2 : 1;
-    static constexpr size_t SMEM = EXCH + ABUFS * ASZ + 64;         // + TMEM address slot
-    // TMEM: 2V columns per thread; the warps of one lane quadrant sit side by side
-    static constexpr int TCOLS = 2 * V;
+    // Spare elements: one per V in the inverse transform (Stockham strides of V and its powers).  In
+    // the forward transforms 8 lanes hold 8 / WP neighbouring threads, of different regions at the
+    // same element where there are as many regions, for which an odd distance of the regions is enough.
+    static constexpr int D = V, DF = MY * WP >= 8 ? 0 : V;
+    static constexpr int RST = (tmfft::pad_at<DF>(L) + 3) / 4 * 4 + (MY == 2 ? 2 : MY == 3 ? 3 : 1);
+    static constexpr int CS = (MY * RST > tmfft::pad_at<D>(Y)) ? MY * RST : tmfft::pad_at<D>(Y);
+    static constexpr size_t EXCH = sizeof(float4) * WP * CS;
+    static constexpr size_t ASZ = sizeof(float4) * T * WP;          // one A staging buffer
+    // the transforms' stage tables, then the pruned forward's factors w0, w1 per butterfly
+    static constexpr int FTAB = tmfft::stage_table_len<L, V>(), TAB = FTAB + tmfft::stage_table_len<Y, V>();
+    static constexpr size_t TABS = (sizeof(float2) * TAB + 15) / 16 * 16 + sizeof(float4) * P;
+    static constexpr int ABUFS = (EXCH + TABS + 2 * ASZ + 64 <= 232448) ? 2 : 1;
+    static constexpr size_t SMEM = EXCH + ABUFS * ASZ + TABS + 64;  // + TMEM address slot, schedule
+    // TMEM: 4V columns per thread; the warps of one lane quadrant sit side by side
+    static constexpr int TCOLS = 4 * V;
     static constexpr uint32_t TMEM_COLS = [] {
-        const int need = ((FULL_WARPS + 3) / 4) * TCOLS * G;
+        const int need = (NT / 32 + 3) / 4 * TCOLS;
         uint32_t n = 32;
         while ((int)n < need) n *= 2;
         return n;
     }();
+    // resident blocks per SM: 128 registers per thread, shared memory, TMEM
+    static constexpr int BPS = [] {
+        int n = 512 / NT;
+        if (n * (SMEM + 1024) > 233472) n = (int)(233472 / (SMEM + 1024));
+        if (n * (int)TMEM_COLS > 512) n = 512 / (int)TMEM_COLS;
+        return n < 1 ? 1 : n;
+    }();
+    // the addresses of radix-18 exchanges are worked out for each item where registers are few: kept
+    // over the items they spill (256 x 3888, 32 orientations: 1.55 ms, 1.46 so; where they fit, a few percent
+    // are lost)
+    static constexpr bool ADDRESSES_ANEW = V == 18 && NT * BPS > 384;
     static_assert(L > 0 && Y % V == 0 && P % PT == 0, "no pruned plan for this template and height");
     static_assert(NT <= 1024 && SMEM <= 232448, "pass B block exceeds the per-block limits");
     static_assert(TMEM_COLS <= 512, "pass B TMEM layout exceeds 512 columns");
-    static_assert(V == 16 || V == 18 || V == 32, "TMEM load sequence covers 16, 18 or 32 values");
-    static_assert(NH == 1 || (NTH % 32 == 0 && W % NH == 0), "halves must be whole warps and whole columns");
+    static_assert(V == 16 || V == 18, "TMEM load sequence covers 16 or 18 values");
 };
-
-// I' values of one thread (V complex, 2V floats) into its TMEM columns
-template <int V>
-__device__ __forceinline__ void tmem_put_values(uint32_t taddr, const float* f) {
-    tmptx::tmem_st16(taddr, f);
-    tmptx::tmem_st16(taddr + 16, f + 16);
-    if constexpr (V == 18) tmptx::tmem_st4(taddr + 32, f + 32);
-    if constexpr (V == 32) {
-        tmptx::tmem_st16(taddr + 32, f + 32);
-        tmptx::tmem_st16(taddr + 48, f + 48);
-    }
-}
 
 // RB = 0: FP32 complex, tiled (c_index).  RB > 0 (the FP16 form): C in FP16
 // complex times 2^half_scale_exp, rows interleaved in blocks of RB,
-// C16[o][y / RB][kx][y % RB], so that a warp's stores (8 consecutive rows of 4
-// columns) fill whole 32-byte sectors and the tensor-core row pass reads a
+// C16[o][y / RB][kx][y % RB], so that a warp's stores (16 consecutive rows of a
+// column) fill whole 32-byte sectors and the tensor-core row pass reads a
 // block of RB rows with one bulk copy.
 template <int T, int Y, int RB = 0>
-__global__ void __launch_bounds__(PassB<T, Y>::NT, 1)
+__global__ void __launch_bounds__(PassB<T, Y>::NT, PassB<T, Y>::BPS)
 k_pass_b(BatchArgs a, int ngroups) {
     using PB = PassB<T, Y>;
-    constexpr int W = PB::W, MY = PB::MY, PT = PB::PT, NT = PB::NT, V = PB::V, P = PB::P, L = PB::L;
+    using tmfft::Pair;
+    constexpr int W = PB::W, WP = PB::WP, MY = PB::MY, PT = PB::PT, NT = PB::NT, V = PB::V, P = PB::P, L = PB::L;
     const int XP = a.XP;
     extern __shared__ __align__(16) unsigned char smem_b[];
-    float2* exch = reinterpret_cast<float2*>(smem_b);
-    float2* abuf = reinterpret_cast<float2*>(smem_b + PB::EXCH);
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem_b + PB::EXCH + PB::ABUFS * PB::ASZ);
-    volatile ColSchedule* sch = reinterpret_cast<volatile ColSchedule*>(smem_b + PB::EXCH + PB::ABUFS * PB::ASZ + 16);
+    float4* exch = reinterpret_cast<float4*>(smem_b);
+    float4* abuf = reinterpret_cast<float4*>(smem_b + PB::EXCH);
+    float4* w01 = reinterpret_cast<float4*>(smem_b + PB::EXCH + PB::ABUFS * PB::ASZ);
+    float2* tab = reinterpret_cast<float2*>(w01 + P);
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem_b + PB::SMEM - 64);
+    volatile ColSchedule* sch = reinterpret_cast<volatile ColSchedule*>(smem_b + PB::SMEM - 48);
     const int tid = threadIdx.x;
     const int warp = tid >> 5;
-    const bool tmem_warp = warp < PB::FULL_WARPS;   // uniform per warp
-    constexpr int NH = PB::NH, WL = PB::WL, NTH = PB::NTH;
-    // half h owns columns h*WL .. h*WL + WL - 1; within it thread = c' + WL*j
-    const int h = tid / NTH, loc = tid % NTH;
-    const int c = h * WL + loc % WL, j = loc / WL;
-    const int s = j % MY, tp = j / MY;
-    constexpr int G = PB::G, WG = PB::WG;
-    // the barrier over the threads that share this thread's columns
-    auto sync = [h]() {
-        if constexpr (NH == 1) __syncthreads();
-        else asm volatile("bar.sync %0, %1;" ::"r"(1 + h), "n"(NTH) : "memory");
-    };
+    const bool act = PB::NA == NT || tid < PB::NA;
+    const int cp = tid % WP, j0 = act ? tid / WP : P - 1;   // column pair, butterfly
+    auto sync = [] { __syncthreads(); };
     if (tid == 0) {
         const ColSchedule cs(ngroups, a.nb, blockIdx.x, gridDim.x);
         sch->nb = cs.nb; sch->nblk = cs.nblk; sch->b = cs.b; sch->rounds = cs.rounds;
-        sch->tail_g = cs.tail_g; sch->o_lo = cs.o_lo; sch->n = cs.n;
+        sch->tail = cs.tail; sch->n = cs.n;
     }
     __syncthreads();
     const int n_items = sch->n;
@@ -568,43 +550,48 @@ k_pass_b(BatchArgs a, int ngroups) {
         tmptx::tmem_alloc(tmem_slot, PB::TMEM_COLS);
         tmptx::tmem_relinquish();
     }
+    tmfft::fill_stage_table<L, V>(tab, a.twy, tid, NT);
+    tmfft::fill_stage_table<Y, V>(tab + PB::FTAB, a.twy, tid, NT);
+    for (int i = tid; i < P; i += NT) {
+        // twiddles of the pruned forward, W_Y^(s * (tp + PT*r)) = w0 * w1^r
+        const float2 w0 = a.twy.template w<-1>((i % MY) * (i / MY), Y), w1 = a.twy.template w<-1>((i % MY) * PT, Y);
+        w01[i] = make_float4(w0.x, w0.y, w1.x, w1.y);
+    }
     tmptx::tmem_fence_before_sync();
     __syncthreads();
     tmptx::tmem_fence_after_sync();
-    const uint32_t tmem = *tmem_slot + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)(PB::TCOLS * G * (warp >> 2));
-    // the item's T rows of A into dst[row][WG]: each half copies (and later
-    // reads) only its own columns
-    constexpr int WGH = WG / NH;   // the item's columns per half
-    auto issue_rows = [&](int it, float2* dst) {
+    const uint32_t tmem = *tmem_slot + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)(PB::TCOLS * (warp >> 2));
+    // the item's T rows of A into dst[row][column pair]
+    auto issue_rows = [&](int it, float4* dst) {
         int grp, oo;
         ColSchedule::locate(sch, it, grp, oo);
-        const float2* src = a.A + (size_t)oo * T * XP + grp * WG + h * WGH;
-        for (int e = loc; e < T * WGH; e += NTH) {
-            const int row = e / WGH, cc = e % WGH;
-            tmptx::cp_async8(dst + row * WG + h * WGH + cc, src + (size_t)row * XP + cc);
-        }
+        const float2* src = a.A + (size_t)oo * T * XP + grp * W;
+        for (int e = tid; e < T * WP; e += NT)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(tmptx::smem_u32(dst + e)),
+                         "l"(src + (size_t)(e / WP) * XP + 2 * (e % WP))
+                         : "memory");
     };
     if (PB::ABUFS == 2) {
         issue_rows(0, abuf);
         tmptx::cp_async_commit();
     }
+    float4* const colbuf = exch + cp;
     int cur_group = -1;
+#pragma unroll 1
     for (int it = 0; it < n_items; it++) {
-        const int kk = it;
-        const float2* acur = abuf + (PB::ABUFS == 2 ? (kk & 1) : 0) * (T * WG);
-        float2* anext = abuf + (PB::ABUFS == 2 ? ((kk + 1) & 1) : 0) * (T * WG);
+        const float4* acur = abuf + (PB::ABUFS == 2 ? (it & 1) : 0) * (T * WP) + cp;
+        float4* anext = abuf + (PB::ABUFS == 2 ? ((it + 1) & 1) : 0) * (T * WP);
         int group, o;
         ColSchedule::locate(sch, it, group, o);
-        const int kx0 = group * WG;
-        // twiddles of the pruned forward, W_Y^(s * (tp + PT*r)) = w0 * w1^r, loaded early
-        // (with 32 values, from the table again every 8 values)
-        const float2 w0 = a.twy.template w<-1>(s * tp, Y);
-        const float2 w1 = a.twy.template w<-1>(s * PT, Y);
+        const int kx = group * W + 2 * cp;
+        int j = j0;
+        if constexpr (PB::ADDRESSES_ANEW) asm volatile("" : "+r"(j));
+        const int s = j % MY, tp = j / MY;   // residue of the pruned forward, its butterfly
+        float4* const fwdbuf = colbuf + s * PB::RST * WP;
         // The buffer the next rows go into was last read at the start of the
         // previous item's forward transform, whose barriers every thread has
-        // passed; the exchange buffers are guarded by the transforms' own barriers.
+        // passed; the exchange buffer is guarded by the transforms' own barriers.
         // With a single staging buffer the rows are reloaded in place, after a barrier.
-        // (Each half copies and reads only its own columns, so its own barrier suffices.)
         if (PB::ABUFS == 1) sync();
         if (PB::ABUFS == 2) {
             if (it + 1 < n_items) issue_rows(it + 1, anext);
@@ -615,105 +602,104 @@ k_pass_b(BatchArgs a, int ngroups) {
             tmptx::cp_async_commit();
             tmptx::cp_async_wait<0>();
         }
-        sync();  // this item's rows of A are visible to every thread of the half
-        if (group != cur_group && tmem_warp) {
-            // the V I' values this thread multiplies with in each chunk of the
-            // group, into its TMEM columns
+        sync();  // this item's rows of A are visible to every thread
+        if (group != cur_group) {
+            // the V I' values of each of this thread's columns, k = j + P r, as column pairs of
+            // the real and the imaginary parts
+            const float2* Ig = a.Ip + (size_t)j * XP + kx;
+            auto fetch = [&](float* f, int r) {
+                const float4 iv = __ldg(reinterpret_cast<const float4*>(Ig + (size_t)P * r * XP));
+                f[0] = iv.x;
+                f[1] = iv.z;
+                f[2] = iv.y;
+                f[3] = iv.w;
+            };
 #pragma unroll 1
-            for (int g = 0; g < G; g++) {
-                const float2* Ig = a.Ip + kx0 + g * W + c;
-                float buf[2 * V];
+            for (int h = 0; h < 4; h++) {
+                float ib[16];
 #pragma unroll
-                for (int r = 0; r < V; r++) {
-                    const float2 iv = __ldg(Ig + (size_t)(j + P * r) * XP);
-                    buf[2 * r] = iv.x;
-                    buf[2 * r + 1] = iv.y;
-                }
-                tmem_put_values<V>(tmem + g * PB::TCOLS, buf);
+                for (int r = 0; r < 4; r++) fetch(ib + 4 * r, 4 * h + r);
+                tmptx::tmem_st16(tmem + 16 * h, ib);
+            }
+            if constexpr (V == 18) {
+                float ib[8];
+                fetch(ib, 16);
+                fetch(ib + 4, 17);
+                tmptx::tmem_st8(tmem + 64, ib);
             }
             tmptx::tmem_wait_st();
+            cur_group = group;
         }
-        cur_group = group;
-#pragma unroll 1
-        for (int g = 0; g < G; g++) {
-            const int col = g * W + c;   // column within the item
-            float2* colbuf = exch + col * PB::CS;
-            float2* fwdbuf = colbuf + s * PB::RST;
-            const uint32_t tslot = tmem + g * PB::TCOLS;
-            float2 v[V];
-            {
-                float2 w = w0;
+        Pair v[V];
+        {
+            const float4 ww = w01[j];
+            float2 w = make_float2(ww.x, ww.y);
+            const float2 w1 = make_float2(ww.z, ww.w);
 #pragma unroll
-                for (int r = 0; r < V; r++) {
-                    if (V == 32 && r % 8 == 0 && r > 0) w = a.twy.template w<-1>(s * (tp + PT * r), Y);
-                    const int n = tp + PT * r;   // rows n >= T of the L-point input are zero
-                    v[r] = (L == T || n < T) ? cmul(acur[n * WG + col], w) : make_float2(0.f, 0.f);
-                    w = cmul(w, w1);
-                }
-            }
-            // every thread passed the item barrier since the buffers were last read
-            tmfft::fft<L, V, -1, false>(v, tp, fwdbuf, a.twy, sync);
-            // thread (s, tp) holds F[k], k = s + MY*(tp + PT*r) = j + P*r
-            if (tmem_warp) {
-                float iv[16];
-                tmptx::tmem_ld16(tslot, iv);
-                tmptx::tmem_wait_ld();
-                float iw[16], ix[4];
-                tmptx::tmem_ld16(tslot + 16, iw);   // in flight while the first values are multiplied
-                if constexpr (V == 18) tmptx::tmem_ld4(tslot + 32, ix);
-#pragma unroll
-                for (int r = 0; r < 8; r++) v[r] = cmul_conj(make_float2(iv[2 * r], iv[2 * r + 1]), v[r]);
-                tmptx::tmem_wait_ld();
-                if constexpr (V == 32) tmptx::tmem_ld16(tslot + 32, iv);
-#pragma unroll
-                for (int r = 0; r < 8; r++) v[8 + r] = cmul_conj(make_float2(iw[2 * r], iw[2 * r + 1]), v[8 + r]);
-                if constexpr (V == 18) {
-                    v[16] = cmul_conj(make_float2(ix[0], ix[1]), v[16]);
-                    v[17] = cmul_conj(make_float2(ix[2], ix[3]), v[17]);
-                }
-                if constexpr (V == 32) {
-                    tmptx::tmem_wait_ld16(iv);
-                    tmptx::tmem_ld16(tslot + 48, iw);
-#pragma unroll
-                    for (int r = 0; r < 8; r++) v[16 + r] = cmul_conj(make_float2(iv[2 * r], iv[2 * r + 1]), v[16 + r]);
-                    tmptx::tmem_wait_ld16(iw);
-#pragma unroll
-                    for (int r = 0; r < 8; r++) v[24 + r] = cmul_conj(make_float2(iw[2 * r], iw[2 * r + 1]), v[24 + r]);
-                }
-            } else {
-                const float2* Ic = a.Ip + kx0 + col;
-#pragma unroll
-                for (int r = 0; r < V; r++) v[r] = cmul_conj(__ldg(Ic + (size_t)(j + P * r) * XP), v[r]);
-            }
-            tmfft::fft<Y, V, +1>(v, j, colbuf, a.twy, sync);
-            if constexpr (RB > 0) {
-                static_assert(G == 1 && Y % RB == 0 && (P % RB == 0), "FP16 output needs whole-column chunks");
-                // row j + P r sits in block j / RB + r P / RB at position j % RB (RB divides P)
-                const float sc = __int_as_float((127 + a.half_scale_exp) << 23);   // 2^e
-                __half2* Co = reinterpret_cast<__half2*>(a.C) + (size_t)o * Y * XP +
-                              ((size_t)(j / RB) * XP + kx0 + col) * RB + (j % RB);
-#pragma unroll
-                for (int r = 0; r < V; r++) {   // streaming stores, as the FP32 output
-                    const __half2 hv = __floats2half2_rn(v[r].x * sc, v[r].y * sc);
-                    __stcs(reinterpret_cast<unsigned int*>(Co + (size_t)r * P * XP), *reinterpret_cast<const unsigned int*>(&hv));
-                }
-            } else if constexpr (G == 1) {
-#pragma unroll
-                for (int r = 0; r < V; r++) __stcs(a.C + c_index<Y>(o, j + P * r, kx0 + col, XP), v[r]);   // streaming
-            } else {
-                sync();   // every thread has read its last-stage inputs from colbuf
-#pragma unroll
-                for (int r = 0; r < V; r++) colbuf[tmfft::pad16(j + P * r)] = v[r];
+            for (int r = 0; r < V; r++) {
+                const int n = tp + PT * r;   // rows n >= T of the L-point input are zero
+                const bool in = L == T || n < T;
+                const float4 f = acur[(in ? n : 0) * WP];
+                const Pair x = tmfft::pmul({make_float2(f.x, f.z), make_float2(f.y, f.w)}, w);
+                v[r] = in ? x : Pair{make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+                w = cmul(w, w1);
             }
         }
-        if constexpr (G > 1) {
-            // the item's 4 columns: whole tiles
-            static_assert(WG == 4, "chunks written together are one tile wide");
-            sync();
-            for (int e = tid; e < Y * WG; e += NT) {
-                const int row = e / WG, cc = e % WG;
-                __stcs(a.C + c_index<Y>(o, row, kx0 + cc, XP), exch[cc * PB::CS + tmfft::pad16(row)]);   // streaming
+        // every thread passed the item barrier since the buffer was last read
+        tmfft::pfft<L, V, -1, WP, PB::DF, false>(v, tp, fwdbuf, tab, act, sync);
+        // thread (s, tp) holds F[k], k = s + MY*(tp + PT*r) = j + P*r
+        {
+            float iv[16], iw[16];
+            auto mul = [&](int r, const float* f) {
+                v[r] = tmfft::pmul_conj(make_float2(f[0], f[1]), make_float2(f[2], f[3]), v[r]);
+            };
+            tmptx::tmem_ld16(tmem, iv);
+            tmptx::tmem_wait_ld16(iv);
+            tmptx::tmem_ld16(tmem + 16, iw);   // in flight while the first values are multiplied
+#pragma unroll
+            for (int r = 0; r < 4; r++) mul(r, iv + 4 * r);
+            tmptx::tmem_wait_ld16(iw);
+            tmptx::tmem_ld16(tmem + 32, iv);
+#pragma unroll
+            for (int r = 0; r < 4; r++) mul(4 + r, iw + 4 * r);
+            tmptx::tmem_wait_ld16(iv);
+            tmptx::tmem_ld16(tmem + 48, iw);
+#pragma unroll
+            for (int r = 0; r < 4; r++) mul(8 + r, iv + 4 * r);
+            tmptx::tmem_wait_ld16(iw);
+            if constexpr (V == 18) tmptx::tmem_ld8(tmem + 64, iv);
+#pragma unroll
+            for (int r = 0; r < 4; r++) mul(12 + r, iw + 4 * r);
+            if constexpr (V == 18) {
+                tmptx::tmem_wait_ld16(iv);
+                mul(16, iv);
+                mul(17, iv + 4);
             }
+        }
+        tmfft::pfft<Y, V, +1, WP, PB::D>(v, j, colbuf, tab + PB::FTAB, act, sync);
+        if (!act) continue;
+        if constexpr (RB > 0) {
+            static_assert(Y % RB == 0 && (P % RB == 0), "a thread's rows sit at one position of their blocks");
+            // row j + P r sits in block j / RB + r P / RB at position j % RB (RB divides P)
+            const float sc = __int_as_float((127 + a.half_scale_exp) << 23);   // 2^e
+            __half2* Co = reinterpret_cast<__half2*>(a.C) + (size_t)o * Y * XP + ((size_t)(j / RB) * XP + kx) * RB + (j % RB);
+#pragma unroll
+            for (int r = 0; r < V; r++) {   // streaming stores, as the FP32 output
+                const __half2 h0 = __floats2half2_rn(v[r].re.x * sc, v[r].im.x * sc);
+                const __half2 h1 = __floats2half2_rn(v[r].re.y * sc, v[r].im.y * sc);
+                __stcs(reinterpret_cast<unsigned int*>(Co + (size_t)r * P * XP), *reinterpret_cast<const unsigned int*>(&h0));
+                __stcs(reinterpret_cast<unsigned int*>(Co + (size_t)r * P * XP + RB), *reinterpret_cast<const unsigned int*>(&h1));
+            }
+        } else {
+            // Rows that a whole number of tiles lies between are that many rows of XP apart: the
+            // rows of even r from the first's place, those of odd r from the second's
+            static_assert(2 * P % c_tile_rows(Y) == 0, "every second row of a thread sits at one position of its tile");
+            float2* const C0 = a.C + c_index<Y>(o, j, kx, XP);
+            float2* const C1 = P % c_tile_rows(Y) == 0 ? C0 + (size_t)P * XP : a.C + c_index<Y>(o, j + P, kx, XP);
+#pragma unroll
+            for (int r = 0; r < V; r++)   // streaming; a warp writes whole tiles
+                __stcs(reinterpret_cast<float4*>((r % 2 ? C1 : C0) + (size_t)(r / 2) * 2 * P * XP),
+                       make_float4(v[r].re.x, v[r].im.x, v[r].re.y, v[r].im.y));
         }
     }
     tmptx::cp_async_wait<0>();
@@ -1532,6 +1518,14 @@ inline cudaError_t c_tensor_maps(CMaps* maps, float2* C, int XP, int Y, int cap)
     return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
 }
 
+// several resident blocks need the largest shared-memory carveout
+template <class K>
+cudaError_t configure_cols(K kernel, size_t smem) {
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared);
+}
+
 // --------------------------------------------------------------------------------------
 // Launch shapes of one geometry, shared by every entry point.
 template <int T, int X, int Y>
@@ -1541,11 +1535,11 @@ struct Launch {
     static_assert(Y % PC::ROWS == 0, "pass C blocks hold whole groups of rows");
     using SC = SliceCol<T>;
     using RC = RowC2R<T>;
-    static constexpr int pass_b_width = PB::WG;   // row pitch alignment (columns)
+    static constexpr int pass_b_width = PB::W;   // row pitch alignment (columns)
     // 4096-high micrographs with 256-row pruned transforms: the residue-grouped column pass
     static constexpr bool RG = (T == 256 && Y == 4096);
     static cudaError_t configure_b() {
-        cudaError_t e = cudaFuncSetAttribute(k_pass_b<T, Y>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PB::SMEM);
+        cudaError_t e = configure_cols(k_pass_b<T, Y>, PB::SMEM);
         if (RG && e == cudaSuccess)
             e = cudaFuncSetAttribute(k_pass_b_rg, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PassBRg::SMEM);
         return e;
@@ -1563,11 +1557,11 @@ struct Launch {
         k_pass_a<T, X><<<dim3(T, a.nb), X / 16, 0, s>>>(a);
     }
     static void pass_b(BatchArgs& a, const CMaps& cmaps, cudaStream_t s, int nsm) {
-        const int ngroups = a.XP / PB::WG;
+        const int ngroups = a.XP / (RG ? 4 : PB::W);
         if (RG && ColSchedule::max_items(ngroups, a.nb, nsm) <= PassBRg::MAX_ITEMS)
             k_pass_b_rg<<<nsm, PassBRg::NT, PassBRg::SMEM, s>>>(a, cmaps.columns, ngroups);
         else
-            k_pass_b<T, Y><<<nsm, PB::NT, PB::SMEM, s>>>(a, ngroups);
+            k_pass_b<T, Y><<<PB::BPS * nsm, PB::NT, PB::SMEM, s>>>(a, ngroups);
     }
     static void pass_c(BatchArgs& a, const CMaps& cmaps, cudaStream_t s, int nsm) {
         const int nblocks = Y / PC::ROWS, resident = PC::MIN_BLOCKS * nsm;
@@ -1602,7 +1596,7 @@ struct LaunchTc {
                 e = cudaFuncSetAttribute(k_pass_b_tc<T, R>, cudaFuncAttributePreferredSharedMemoryCarveout,
                                          (int)cudaSharedmemCarveoutMaxShared);
         } else
-            e = cudaFuncSetAttribute(k_pass_b<T, Y, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PB::SMEM);
+            e = configure_cols(k_pass_b<T, Y, R>, PB::SMEM);
         if (e != cudaSuccess) return e;
         return cudaFuncSetAttribute(k_pass_c_tc<X>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PCT::smem_bytes(XP, bins));
     }
@@ -1611,7 +1605,7 @@ struct LaunchTc {
             // items = (group of 4 columns, orientation); two blocks per SM
             k_pass_b_tc<T, R><<<2 * nsm, PBT::NT, PBT::SMEM, s>>>(a, a.XP / 4, tabs + rows_tab_bytes / 16);
         } else {
-            k_pass_b<T, Y, R><<<nsm, PB::NT, PB::SMEM, s>>>(a, a.XP / PB::WG);
+            k_pass_b<T, Y, R><<<PB::BPS * nsm, PB::NT, PB::SMEM, s>>>(a, a.XP / PB::W);
         }
     }
     static void pass_c(BatchArgs& a, cudaStream_t s, const uint4* dft) {
