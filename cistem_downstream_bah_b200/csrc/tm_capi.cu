@@ -67,6 +67,7 @@ struct tm_ctx {
     double* rowstat = nullptr;
     float* mip = nullptr;
     int* best = nullptr;
+    int* best_parts = nullptr;   // the row pass's divided batches (BatchArgs)
     double *sum = nullptr, *sumsq = nullptr;
     unsigned long long* hist = nullptr;
     int* err_flag = nullptr;
@@ -152,6 +153,7 @@ struct Variant {
     WhitenFn whiten;
     int (*run_batch_images)(tm_ctx*, tmk::BatchArgs&, const int* ids, int n_ids);   // image-set batch
     const TensorForm* tc;   // null where the FP16 tensor-core form has no kernels
+    int (*pass_c_parts)(int nsm);   // most blocks that share a batch in the row pass (null: one)
 };
 
 // number of points of the whitening curve (match_template.cpp:702)
@@ -424,11 +426,13 @@ struct GenImpl {
 
 #define TM_VARIANT(T, X, Y)                                                                                 \
     {T, X, Y, tmk::Launch<T, X, Y>::pass_b_width, &Impl<T, X, Y>::run_batch, &Impl<T, X, Y>::configure,          \
-     &Impl<T, X, Y>::run_stages, &whiten_on_device<X, Y>, &Impl<T, X, Y>::run_batch_images, nullptr}
+     &Impl<T, X, Y>::run_stages, &whiten_on_device<X, Y>, &Impl<T, X, Y>::run_batch_images, nullptr,       \
+     &tmk::Launch<T, X, Y>::pass_c_parts}
 // a geometry that also has the FP16 tensor-core form
 #define TM_VARIANT_TC(T, X, Y)                                                                              \
     {T, X, Y, tmk::Launch<T, X, Y>::pass_b_width, &Impl<T, X, Y>::run_batch, &Impl<T, X, Y>::configure,          \
-     &Impl<T, X, Y>::run_stages, &whiten_on_device<X, Y>, &Impl<T, X, Y>::run_batch_images, &TcImpl<T, X, Y>::form}
+     &Impl<T, X, Y>::run_stages, &whiten_on_device<X, Y>, &Impl<T, X, Y>::run_batch_images, &TcImpl<T, X, Y>::form, \
+     &tmk::Launch<T, X, Y>::pass_c_parts}
 
 // Geometries with compiled kernels: template box T on a padded X x Y
 // micrograph.  X is a power of two (the reference turns a micrograph whose
@@ -537,7 +541,7 @@ int wait_stream(tm_ctx* c, double limit_s) {
 
 void free_all(tm_ctx* c) {
     void* ptrs[] = {c->tmpl, c->Ip, c->S, c->A, c->C, c->norm, c->twx, c->twy, c->twt, c->P, c->filter, c->rot,
-                    c->rowstat, c->mip, c->best, c->sum, c->sumsq, c->hist, c->err_flag, c->dft};
+                    c->rowstat, c->mip, c->best, c->best_parts, c->sum, c->sumsq, c->hist, c->err_flag, c->dft};
     for (void* p : ptrs)
         if (p) cudaFree(p);
     for (tm_ctx::Slot& sl : c->slots) {
@@ -708,6 +712,7 @@ tmk::BatchArgs make_args(tm_ctx* c) {
     a.Ip = c->Ip;
     a.mip = c->mip;
     a.best = c->best;
+    a.best_parts = c->best_parts;
     a.sum = c->sum;
     a.sumsq = c->sumsq;
     a.hist = c->hist;
@@ -1036,6 +1041,8 @@ int tm_create(const tm_dims* dims, tm_ctx** out) {
     TRY(dalloc(c, &c->filter, T * TP));
     TRY(dalloc(c, &c->mip, X * Y));
     TRY(dalloc(c, &c->best, X * Y));
+    if (c->var->pass_c_parts && c->var->pass_c_parts(c->nsm) > 1)
+        TRY(dalloc(c, &c->best_parts, (size_t)(c->var->pass_c_parts(c->nsm) - 1) * X * Y));
     TRY(dalloc(c, &c->sum, X * Y));
     TRY(dalloc(c, &c->sumsq, X * Y));
     TRY(dalloc(c, &c->hist, (size_t)1024));

@@ -100,6 +100,7 @@ struct BatchArgs {
     const float2* Ip;             // Y * XP prepared micrograph spectrum
     float* mip;                   // Y * X
     int* best;                    // Y * X
+    int* best_parts;              // best of a divided batch's parts 1, 2, ...: kPassCParts - 1 planes of Y * X (or null)
     double* sum;                  // Y * X
     double* sumsq;                // Y * X
     unsigned long long* hist;     // hist_bins
@@ -1068,6 +1069,15 @@ __host__ __device__ inline int hist_copies(int bins, int max_copies) {
 // FP64 running sums once per batch.  Columns 64-127 hold the thread's twiddle
 // multipliers.  The best orientation is written to memory when a pixel's
 // maximum changes (the n-th orientation changes it with probability 1/n) and never read.
+//
+// Small images have too few rows for the chip (512 x 512: 128 blocks of four rows, one or none per SM, each
+// waiting for its own latencies: 206 us for 256 orientations): PARTS blocks of a cluster then share a group of
+// rows, each with a part of the batch.  Every part starts from the maxima so far and
+// keeps its own best orientations; at the end each block merges a share of the pixels over the parts' shared
+// memory, in the order of the orientations (a later part has to exceed the earlier ones).
+// 512 x 512, 256 orientations: 206 -> 126 us (101 at the rate of 4096 x 4096); 256 x 256, 32 on one block per eight rows
+// 35 us, 128 on eight 34.
+constexpr int kPassCParts = 8;
 template <int X>
 struct PassC {
     static constexpr int H = X / 2;
@@ -1083,6 +1093,12 @@ struct PassC {
     static constexpr int WCOLS = 128;
     static constexpr uint32_t TMEM_COLS = WCOLS * ((NT / 32 + 3) / 4);   // warps of a lane quadrant side by side
     static_assert(PL::radix(0) == 8 && PL::radix(1) == 8 && (PL::stages == 3 || PL::stages == 4) && G <= 32, "pass C widths");
+    // blocks that share a group of rows of an image of height Y: as many as are resident together
+    static int parts(int Y, int nsm) {
+        int n = 1;
+        while (n < kPassCParts && Y / ROWS * 2 * n <= MIN_BLOCKS * nsm) n *= 2;
+        return n;
+    }
     // dynamic shared memory for a row pitch XP and `bins` histogram bins (one word for values outside)
     static size_t smem_bytes(int XP, int bins) {
         return 128 + sizeof(float2) * (size_t)ROWS * 2 * c_row_len(XP) + sizeof(float4) * 2 * (size_t)ROWS * EXL + 4 * ((size_t)bins + 1);
@@ -1156,9 +1172,10 @@ struct PassCTw {
     }
 };
 
-template <int X>
+// DIVIDED: the `parts` blocks of a cluster share a group of rows (a group per cluster).
+template <int X, bool DIVIDED = false>
 __global__ void __launch_bounds__(PassC<X>::NT, PassC<X>::MIN_BLOCKS)
-k_pass_c(BatchArgs a, const __grid_constant__ CUtensorMap cmap, int Y) {
+k_pass_c(BatchArgs a, const __grid_constant__ CUtensorMap cmap, int Y, int parts) {
     using PC = PassC<X>;
     using PL = typename PC::PL;
     using TW = PassCTw<X>;
@@ -1175,7 +1192,13 @@ k_pass_c(BatchArgs a, const __grid_constant__ CUtensorMap cmap, int Y) {
     const int tid = threadIdx.x, warp = tid >> 5;
     const int t = tid % P, rl = tid / P;
     const int l = t % G, j = t / G;   // lane and group of the stages after the first
-    const int npairs = (a.nb + 1) >> 1, nblocks = Y / ROWS;
+    const int nblocks = Y / ROWS;
+    // this block's rows and pairs of orientations
+    const int part = DIVIDED ? (int)blockIdx.x % parts : 0, rb0 = DIVIDED ? (int)blockIdx.x / parts : (int)blockIdx.x;
+    const int rbstep = DIVIDED ? nblocks : (int)gridDim.x;
+    const int i0 = DIVIDED ? part * ((a.nb + 1) >> 1) / parts : 0;
+    const int npairs = DIVIDED ? (part + 1) * ((a.nb + 1) >> 1) / parts : (a.nb + 1) >> 1;   // pairs i0 .. npairs - 1
+    int* const best = !DIVIDED || part == 0 ? a.best : a.best_parts + (size_t)(part - 1) * Y * X;
     if (tid == 0) tmptx::mbar_init(mbar, 1);
     if (warp == 0) {
         tmptx::tmem_alloc(tmem_slot, PC::TMEM_COLS);
@@ -1201,7 +1224,7 @@ k_pass_c(BatchArgs a, const __grid_constant__ CUtensorMap cmap, int Y) {
                                o < a.nb ? o : 2 * i, mbar);
         }
     };
-    if (warp == 0 && npairs > 0 && (int)blockIdx.x < nblocks) issue_pair(blockIdx.x, 0);
+    if (warp == 0 && npairs > i0 && rb0 < nblocks) issue_pair(rb0, i0);
     {
         // the packing's multipliers W_X^k, k = t + P r (columns 64-79), and those of stages 1, 2, 3
         float z[16];
@@ -1225,7 +1248,7 @@ k_pass_c(BatchArgs a, const __grid_constant__ CUtensorMap cmap, int Y) {
     const unsigned int nbins = (unsigned int)a.hist_bins;
     bool timed_out = false, stop = false;
     uint32_t n = 0;   // pairs done: parity of the barrier's phase and of the exchange buffer
-    for (int rb = blockIdx.x; rb < nblocks && !stop; rb += gridDim.x) {
+    for (int rb = rb0; rb < nblocks && !stop; rb += rbstep) {
     const size_t pix0 = (size_t)rb * ROWS * X;
     float mip[16];
     float fs[16], pq[16];   // plain sums over at most 8 orientations
@@ -1245,7 +1268,7 @@ k_pass_c(BatchArgs a, const __grid_constant__ CUtensorMap cmap, int Y) {
         tmptx::tmem_st16(tcomp + 48, z);
         tmptx::tmem_wait_st();
     }
-    for (int i = 0; i < npairs; i++, n++) {
+    for (int i = i0; i < npairs; i++, n++) {
         float4* const ex = exch + (n & 1) * (ROWS * EXL) + rl * EXL;
         float tb[16];
         tmptx::tmem_ld16(tcomp + 64, tb);
@@ -1290,7 +1313,7 @@ k_pass_c(BatchArgs a, const __grid_constant__ CUtensorMap cmap, int Y) {
         // every thread has read its row values: the next pair's rows may arrive
         if (warp == 0) {
             if (i + 1 < npairs) issue_pair(rb, i + 1);
-            else if (rb + (int)gridDim.x < nblocks) issue_pair(rb + gridDim.x, 0);
+            else if (rb + rbstep < nblocks) issue_pair(rb + rbstep, 0);
         }
         float4* const eg = ex + S * j;
 #pragma unroll
@@ -1333,7 +1356,7 @@ k_pass_c(BatchArgs a, const __grid_constant__ CUtensorMap cmap, int Y) {
             if (changed) {
 #pragma unroll
                 for (int k = 0; k < 4; k++)
-                    if (m[k] > mip[r0 + k]) a.best[pix0 + own + 2 * P * ((r0 + k) / 2) + k % 2] = val(r0 + k).x == m[k] ? g : g + 1;
+                    if (m[k] > mip[r0 + k]) best[pix0 + own + 2 * P * ((r0 + k) / 2) + k % 2] = val(r0 + k).x == m[k] ? g : g + 1;
             }
 #pragma unroll
             for (int k = 0; k < 4; k++) mip[r0 + k] = m[k];
@@ -1363,7 +1386,7 @@ k_pass_c(BatchArgs a, const __grid_constant__ CUtensorMap cmap, int Y) {
                 count(fmaf(p, a.hist_inv_step, hoff));
             }
         }
-        if ((i & 3) == 3 || i == npairs - 1) {
+        if (((i - i0) & 3) == 3 || i == npairs - 1) {
             // Kahan: the compensation holds what the last addition added beyond its input
 #pragma unroll
             for (int sweep = 0; sweep < 4; sweep++) {   // 8 pixels of one sum at a time
@@ -1387,7 +1410,7 @@ k_pass_c(BatchArgs a, const __grid_constant__ CUtensorMap cmap, int Y) {
             tmptx::tmem_wait_st();
         }
     }
-    if (stop) break;
+    if (!DIVIDED && stop) break;
     // the batch's sums into the FP64 running sums, and the maxima, in pixel order through the
     // exchange buffers (one spare element per 16: the strided writes are conflict-free), so that
     // memory is accessed in whole lines with all of a thread's loads in flight
@@ -1409,6 +1432,36 @@ k_pass_c(BatchArgs a, const __grid_constant__ CUtensorMap cmap, int Y) {
         tmptx::tmem_wait_ld32(send);
 #pragma unroll
         for (int r = 0; r < 16; r++) staged[2 * ROWS * EXL + at + px(r)] = (double)send[r] - (double)send[16 + r];
+    }
+    if constexpr (DIVIDED) {
+        // (the maxima in the row buffer, whose last copies have been waited for; after a timeout
+        // they are no results, but the cluster's barriers are passed all the same)
+        float* const maxima = reinterpret_cast<float*>(rows);
+        if (stop) tmptx::mbar_wait_bounded(mbar, n & 1, kWaitLimit);
+#pragma unroll
+        for (int r = 0; r < 16; r++) maxima[at + px(r)] = mip[r];
+        tmptx::cluster_sync();
+        // this block's share of the pixels: PER / parts per thread
+        for (int e = part * PER / parts; e < (part + 1) * PER / parts; e++) {
+            const size_t pix = pix0 + tid + e * NT;
+            const int x = pad(tid + e * NT);
+            double s = a.sum[pix], q = a.sumsq[pix];
+            float m = 0.f;
+            int won = 0;
+            for (int p = 0; p < parts; p++) {
+                s += tmptx::cluster_ld_f64(tmptx::cluster_addr(staged + x, p));
+                q += tmptx::cluster_ld_f64(tmptx::cluster_addr(staged + 2 * ROWS * EXL + x, p));
+                const float mp = tmptx::cluster_ld_f32(tmptx::cluster_addr(maxima + x, p));
+                if (p > 0 && mp > m) won = p;
+                m = p > 0 ? fmaxf(m, mp) : mp;
+            }
+            a.sum[pix] = s;
+            a.sumsq[pix] = q;
+            a.mip[pix] = m;
+            if (won) a.best[pix] = __ldcg(a.best_parts + (size_t)(won - 1) * Y * X + pix);
+        }
+        tmptx::cluster_sync();   // the other blocks have read this one's shared memory
+        break;
     }
     __syncthreads();
 #pragma unroll 1
@@ -1538,6 +1591,9 @@ struct Launch {
     static constexpr int pass_b_width = PB::W;   // row pitch alignment (columns)
     // 4096-high micrographs with 256-row pruned transforms: the residue-grouped column pass
     static constexpr bool RG = (T == 256 && Y == 4096);
+    // images whose row pass divides its batches (PassC::parts)
+    static constexpr bool DIVIDES = 2 * (Y / PC::ROWS) <= PC::MIN_BLOCKS * 160;
+    static int pass_c_parts(int nsm) { return DIVIDES ? PC::parts(Y, nsm) : 1; }
     static cudaError_t configure_b() {
         cudaError_t e = configure_cols(k_pass_b<T, Y>, PB::SMEM);
         if (RG && e == cudaSuccess)
@@ -1547,7 +1603,12 @@ struct Launch {
     static cudaError_t configure(int XP, int bins) {
         const cudaError_t e = configure_b();
         if (e != cudaSuccess) return e;
-        return cudaFuncSetAttribute(k_pass_c<X>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PC::smem_bytes(XP, bins));
+        const int smem = (int)PC::smem_bytes(XP, bins);
+        if constexpr (DIVIDES) {
+            const cudaError_t d = cudaFuncSetAttribute(k_pass_c<X, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+            if (d != cudaSuccess) return d;
+        }
+        return cudaFuncSetAttribute(k_pass_c<X>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     }
     // slice, projection, normalisation and row transforms
     static void prep(BatchArgs& a, cudaStream_t s) {
@@ -1565,7 +1626,28 @@ struct Launch {
     }
     static void pass_c(BatchArgs& a, const CMaps& cmaps, cudaStream_t s, int nsm) {
         const int nblocks = Y / PC::ROWS, resident = PC::MIN_BLOCKS * nsm;
-        k_pass_c<X><<<nblocks < resident ? nblocks : resident, PC::NT, PC::smem_bytes(a.XP, a.hist_bins), s>>>(a, cmaps.rows, Y);
+        const size_t smem = PC::smem_bytes(a.XP, a.hist_bins);
+        if constexpr (DIVIDES) {
+            // at least two pairs of orientations for each part
+            int parts = a.best_parts ? PC::parts(Y, nsm) : 1;
+            while (parts > 1 && a.nb < 4 * parts) parts /= 2;
+            if (parts > 1) {
+                cudaLaunchAttribute cluster;
+                cluster.id = cudaLaunchAttributeClusterDimension;
+                cluster.val.clusterDim.x = parts;
+                cluster.val.clusterDim.y = cluster.val.clusterDim.z = 1;
+                cudaLaunchConfig_t cfg{};
+                cfg.gridDim = dim3(nblocks * parts);
+                cfg.blockDim = dim3(PC::NT);
+                cfg.dynamicSmemBytes = smem;
+                cfg.stream = s;
+                cfg.attrs = &cluster;
+                cfg.numAttrs = 1;
+                cudaLaunchKernelEx(&cfg, k_pass_c<X, true>, a, cmaps.rows, Y, parts);
+                return;
+            }
+        }
+        k_pass_c<X><<<nblocks < resident ? nblocks : resident, PC::NT, smem, s>>>(a, cmaps.rows, Y, 1);
     }
 };
 
