@@ -1194,11 +1194,17 @@ k_pass_c(BatchArgs a, const __grid_constant__ CUtensorMap cmap, int Y, int parts
     const int l = t % G, j = t / G;   // lane and group of the stages after the first
     const int nblocks = Y / ROWS;
     // this block's rows and pairs of orientations
-    const int part = DIVIDED ? (int)blockIdx.x % parts : 0, rb0 = DIVIDED ? (int)blockIdx.x / parts : (int)blockIdx.x;
-    const int rbstep = DIVIDED ? nblocks : (int)gridDim.x;
-    const int i0 = DIVIDED ? part * ((a.nb + 1) >> 1) / parts : 0;
-    const int npairs = DIVIDED ? (part + 1) * ((a.nb + 1) >> 1) / parts : (a.nb + 1) >> 1;   // pairs i0 .. npairs - 1
-    int* const best = !DIVIDED || part == 0 ? a.best : a.best_parts + (size_t)(part - 1) * Y * X;
+    int part = 0, rb0 = blockIdx.x, i0 = 0, npairs = (a.nb + 1) >> 1;   // pairs i0 .. npairs - 1
+    if constexpr (DIVIDED) {
+        part = (int)blockIdx.x % parts;
+        rb0 = (int)blockIdx.x / parts;
+        i0 = part * npairs / parts;
+        npairs = (part + 1) * npairs / parts;
+    }
+    auto best = [&]() -> int* {
+        if constexpr (DIVIDED) return part == 0 ? a.best : a.best_parts + (size_t)(part - 1) * Y * X;
+        else return a.best;
+    };
     if (tid == 0) tmptx::mbar_init(mbar, 1);
     if (warp == 0) {
         tmptx::tmem_alloc(tmem_slot, PC::TMEM_COLS);
@@ -1248,7 +1254,7 @@ k_pass_c(BatchArgs a, const __grid_constant__ CUtensorMap cmap, int Y, int parts
     const unsigned int nbins = (unsigned int)a.hist_bins;
     bool timed_out = false, stop = false;
     uint32_t n = 0;   // pairs done: parity of the barrier's phase and of the exchange buffer
-    for (int rb = rb0; rb < nblocks && !stop; rb += rbstep) {
+    for (int rb = rb0; rb < nblocks && !stop; rb += gridDim.x) {   // (DIVIDED: leaves after the first)
     const size_t pix0 = (size_t)rb * ROWS * X;
     float mip[16];
     float fs[16], pq[16];   // plain sums over at most 8 orientations
@@ -1313,7 +1319,7 @@ k_pass_c(BatchArgs a, const __grid_constant__ CUtensorMap cmap, int Y, int parts
         // every thread has read its row values: the next pair's rows may arrive
         if (warp == 0) {
             if (i + 1 < npairs) issue_pair(rb, i + 1);
-            else if (rb + rbstep < nblocks) issue_pair(rb + rbstep, 0);
+            else if (!DIVIDED && rb + (int)gridDim.x < nblocks) issue_pair(rb + gridDim.x, 0);
         }
         float4* const eg = ex + S * j;
 #pragma unroll
@@ -1356,7 +1362,7 @@ k_pass_c(BatchArgs a, const __grid_constant__ CUtensorMap cmap, int Y, int parts
             if (changed) {
 #pragma unroll
                 for (int k = 0; k < 4; k++)
-                    if (m[k] > mip[r0 + k]) best[pix0 + own + 2 * P * ((r0 + k) / 2) + k % 2] = val(r0 + k).x == m[k] ? g : g + 1;
+                    if (m[k] > mip[r0 + k]) best()[pix0 + own + 2 * P * ((r0 + k) / 2) + k % 2] = val(r0 + k).x == m[k] ? g : g + 1;
             }
 #pragma unroll
             for (int k = 0; k < 4; k++) mip[r0 + k] = m[k];

@@ -71,10 +71,7 @@ __device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.comm
 __device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
 __device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 
-// Ampere-style asynchronous 8-byte copy global -> shared (LDGSTS) and its groups.
-__device__ __forceinline__ void cp_async8(void* dst, const void* src) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
-}
+// groups of cp.async copies (global -> shared)
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
@@ -119,11 +116,6 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float* v) {
         : "r"(taddr)
         : "memory");
 }
-// 32 consecutive 32-bit columns of this thread's lane (as two x16 accesses)
-__device__ __forceinline__ void tmem_st32(uint32_t taddr, const float* v) {
-    tmem_st16(taddr, v);
-    tmem_st16(taddr + 16, v + 16);
-}
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float* v) {
     tmem_ld16(taddr, v);
     tmem_ld16(taddr + 16, v + 16);
@@ -137,18 +129,6 @@ __device__ __forceinline__ void tmem_st8(uint32_t taddr, const float* v) {
 __device__ __forceinline__ void tmem_ld8(uint32_t taddr, float* v) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
                  : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
-                 : "r"(taddr)
-                 : "memory");
-}
-// 4 consecutive 32-bit columns of this thread's lane
-__device__ __forceinline__ void tmem_st4(uint32_t taddr, const float* v) {
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1, %2, %3, %4};" ::"r"(taddr), "f"(v[0]), "f"(v[1]),
-                 "f"(v[2]), "f"(v[3])
-                 : "memory");
-}
-__device__ __forceinline__ void tmem_ld4(uint32_t taddr, float* v) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
-                 : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3])
                  : "r"(taddr)
                  : "memory");
 }
