@@ -1063,11 +1063,11 @@ __host__ __device__ inline int hist_copies(int bins, int max_copies) {
 // and histogram are set up once, and the rows of C of the next pair -- the next rows' first
 // pair after the last -- arrive by tensor-map copies while a pair is transformed.
 //
-// The per-pixel sum and sum of squares are plain FP32 sums over at most 8
-// orientations in registers, added (Kahan) every 8 orientations into
-// compensated FP32 sums in the thread's TMEM columns 0-63 and from there to the
-// FP64 running sums once per batch.  Columns 64-127 hold the thread's twiddle
-// multipliers.  The best orientation is written to memory when a pixel's
+// The per-pixel sum and sum of squares stay in the thread's TMEM columns 0-63 over the
+// batch and go from there to the FP64 running sums.  Below 2048 pixels they are FP64
+// sums of every value (EXACT).  From 2048 on they are plain FP32 sums over at most 8
+// orientations in registers, added (Kahan) every 8 orientations into compensated FP32 sums.
+// Columns 64-127 hold the thread's twiddle multipliers.  The best orientation is written to memory when a pixel's
 // maximum changes (the n-th orientation changes it with probability 1/n) and never read.
 //
 // Small images have too few rows for the chip (512 x 512: 128 blocks of four rows, one or none per SM, each
@@ -1088,6 +1088,12 @@ struct PassC {
     static constexpr int ROWS = P >= 128 ? 1 : 128 / P;
     static constexpr int NT = P * ROWS;             // 128 threads (256 at X = 4096)
     static constexpr int EXL = 8 * S;               // exchange buffer of a row
+    // Widths whose sums take every value by itself: plain FP32 sums over 8 orientations have 2.7 times the
+    // error of sums compensated at each (128 orientations of unit noise: 6.2e-7 against 2.3e-7,
+    // emulated), FP64 has none to speak of.  The conversions share their unit with those of the histogram: 512
+    // orientations at 1024 x 1024 0.81 ms with plain sums, 0.90 so (0.97 with two-term FP32 sums of
+    // each value); 512 x 512 0.287 both; 256 x 256 0.143 and 0.148
+    static constexpr bool EXACT = X < 2048;
     // 512 threads per SM at 128 registers: every block has its 128 TMEM columns per warp
     static constexpr int MIN_BLOCKS = 512 / NT;
     static constexpr int WCOLS = 128;
@@ -1110,6 +1116,13 @@ __device__ __forceinline__ float fmax3(float a, float b, float c) {
     float r;
     asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
     return r;
+}
+
+// a double in two TMEM columns
+__device__ __forceinline__ double f64_of(float lo, float hi) { return __hiloint2double(__float_as_int(hi), __float_as_int(lo)); }
+__device__ __forceinline__ void f64_to(double d, float& lo, float& hi) {
+    lo = __int_as_float(__double2loint(d));
+    hi = __int_as_float(__double2hiint(d));
 }
 
 // Twiddle multipliers of stage s of the row pass's transform in lane l of group j, in 16 TMEM
@@ -1257,13 +1270,11 @@ k_pass_c(BatchArgs a, const __grid_constant__ CUtensorMap cmap, int Y, int parts
     for (int rb = rb0; rb < nblocks && !stop; rb += gridDim.x) {   // (DIVIDED: leaves after the first)
     const size_t pix0 = (size_t)rb * ROWS * X;
     float mip[16];
-    float fs[16], pq[16];   // plain sums over at most 8 orientations
+    float fs[PC::EXACT ? 1 : 16], pq[PC::EXACT ? 1 : 16];   // plain sums over at most 8 orientations
 #pragma unroll
-    for (int r = 0; r < 16; r++) {
-        mip[r] = a.mip[pix0 + own + 2 * P * (r / 2) + r % 2];
-        fs[r] = 0.f;
-        pq[r] = 0.f;
-    }
+    for (int r = 0; r < 16; r++) mip[r] = a.mip[pix0 + own + 2 * P * (r / 2) + r % 2];
+#pragma unroll
+    for (int r = 0; r < (PC::EXACT ? 1 : 16); r++) fs[r] = pq[r] = 0.f;
     {
         float z[16];
 #pragma unroll
@@ -1371,7 +1382,47 @@ k_pass_c(BatchArgs a, const __grid_constant__ CUtensorMap cmap, int Y, int parts
             const unsigned int bin = (unsigned int)__float2int_rz(b);
             atomicAdd(&shist[bin < nbins ? bin : nbins], 1u);
         };
-        if (two) {
+        auto bins = [&](int r) {
+            const float2 p = val(r);
+            if (two) {
+                const float2 b = tmfft::fma2(p, hinv2, hoff2);
+                count(b.x);
+                count(b.y);
+            } else {
+                count(fmaf(p.x, a.hist_inv_step, hoff));
+            }
+        };
+        if constexpr (PC::EXACT) {
+            // FP64 sums of pixel r in columns 2 r (sum) and 32 + 2 r (sum of squares), 4 pixels at a
+            // time, whose bins are counted while the sums arrive
+#pragma unroll
+            for (int h = 0; h < 4; h++) {
+                float sm[8], sq[8];
+                tmptx::tmem_ld8(tcomp + 8 * h, sm);
+                tmptx::tmem_ld8(tcomp + 32 + 8 * h, sq);
+#pragma unroll
+                for (int k = 0; k < 4; k++) bins(4 * h + k);
+                tmptx::tmem_wait_ld8x2(sm, sq);
+#pragma unroll
+                for (int k = 0; k < 4; k++) {
+                    const float2 p = val(4 * h + k);
+                    double ds = f64_of(sm[2 * k], sm[2 * k + 1]), dq = f64_of(sq[2 * k], sq[2 * k + 1]);
+                    const double x = p.x;
+                    ds += x;
+                    dq = fma(x, x, dq);
+                    if (two) {
+                        const double y = p.y;
+                        ds += y;
+                        dq = fma(y, y, dq);
+                    }
+                    f64_to(ds, sm[2 * k], sm[2 * k + 1]);
+                    f64_to(dq, sq[2 * k], sq[2 * k + 1]);
+                }
+                tmptx::tmem_st8(tcomp + 8 * h, sm);
+                tmptx::tmem_st8(tcomp + 32 + 8 * h, sq);
+            }
+            tmptx::tmem_wait_st();
+        } else if (two) {
 #pragma unroll
             for (int r = 0; r < 16; r++) {
                 const float2 p = val(r);
@@ -1379,9 +1430,7 @@ k_pass_c(BatchArgs a, const __grid_constant__ CUtensorMap cmap, int Y, int parts
                 pq[r] = fmaf(p.x, p.x, pq[r]);
                 fs[r] += p.y;
                 pq[r] = fmaf(p.y, p.y, pq[r]);
-                const float2 b = tmfft::fma2(p, hinv2, hoff2);
-                count(b.x);
-                count(b.y);
+                bins(r);
             }
         } else {
 #pragma unroll
@@ -1389,10 +1438,10 @@ k_pass_c(BatchArgs a, const __grid_constant__ CUtensorMap cmap, int Y, int parts
                 const float p = val(r).x;
                 fs[r] += p;
                 pq[r] = fmaf(p, p, pq[r]);
-                count(fmaf(p, a.hist_inv_step, hoff));
+                bins(r);
             }
         }
-        if (((i - i0) & 3) == 3 || i == npairs - 1) {
+        if (!PC::EXACT && (((i - i0) & 3) == 3 || i == npairs - 1)) {
             // Kahan: the compensation holds what the last addition added beyond its input
 #pragma unroll
             for (int sweep = 0; sweep < 4; sweep++) {   // 8 pixels of one sum at a time
@@ -1431,13 +1480,14 @@ k_pass_c(BatchArgs a, const __grid_constant__ CUtensorMap cmap, int Y, int parts
         tmptx::tmem_ld16(tcomp, send);
         tmptx::tmem_ld16(tcomp + 16, send + 16);
         tmptx::tmem_wait_ld32(send);
+        auto sum = [&](int r) { return PC::EXACT ? f64_of(send[2 * r], send[2 * r + 1]) : (double)send[r] - (double)send[16 + r]; };
 #pragma unroll
-        for (int r = 0; r < 16; r++) staged[at + px(r)] = (double)send[r] - (double)send[16 + r];
+        for (int r = 0; r < 16; r++) staged[at + px(r)] = sum(r);
         tmptx::tmem_ld16(tcomp + 32, send);
         tmptx::tmem_ld16(tcomp + 48, send + 16);
         tmptx::tmem_wait_ld32(send);
 #pragma unroll
-        for (int r = 0; r < 16; r++) staged[2 * ROWS * EXL + at + px(r)] = (double)send[r] - (double)send[16 + r];
+        for (int r = 0; r < 16; r++) staged[2 * ROWS * EXL + at + px(r)] = sum(r);
     }
     if constexpr (DIVIDED) {
         // (the maxima in the row buffer, whose last copies have been waited for; after a timeout
