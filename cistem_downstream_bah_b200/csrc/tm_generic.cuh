@@ -260,7 +260,7 @@ k_pass_c_gen(BatchArgs a, int X, int Y, GenPlan ph) {
 // before).  With few warps per SM these kernels wait for memory first of all, so the twiddle
 // table and the next item's input lie in shared memory where they fit.  64 orientations at
 // 2700 x 2700, line by line -> pairs: rows of A 0.74 -> 0.38 ms, columns 6.3 -> 3.9, rows of
-// C 7.0 -> 2.9; what bounds them is the exchange through shared memory once per radix
+// C 7.0 -> 2.5; what bounds them is the exchange through shared memory once per radix
 // (16 bytes per element and stage, in and out).  Where two pairs' buffers do not fit shared
 // memory the one-line forms stay.
 
@@ -431,8 +431,10 @@ __global__ void __launch_bounds__(kGenNT) k_pass_b_gen2(const __grid_constant__ 
 }
 
 // k_pass_c_gen2: block per row y, two orientations at a time; thread t owns the pixels x = t + NT j
-// and keeps their state over the batch: maxima and plain sums over at most 8 orientations
-// in registers, the compensated sums they are added to (as k_pass_c) in TMEM.  An even width
+// and keeps their state over the batch: maxima in registers, FP64 sums of every value in TMEM
+// (the doubles of pixel j in columns 2 j, sum, and 2 MAXP + 2 j, sum of squares; plain FP32 sums over
+// 8 orientations, compensated between the eights, had 6 times the error of sums compensated at each,
+// and their registers spilled: 64 orientations at 2700 x 2700 2.86 ms, 2.51 so).  An even width
 // uses the c2r packing of k_pass_c (an X/2-point inverse FFT whose outputs hold pixel pairs);
 // an odd width (the reference's factorisation can give one, e.g. 3^8) the full X-point
 // inverse of the Hermitian extension, the imaginary part of the DC term ignored as FFTW's
@@ -450,7 +452,7 @@ __global__ void __launch_bounds__(NT, NT == 512 ? 1 : 2)
 k_pass_c_gen2(const __grid_constant__ BatchArgs a, int X, int Y, const __grid_constant__ GenPlan ph) {
     extern __shared__ __align__(16) float4 pbuf[];   // 2 x L, L = X/2 or X
     __shared__ uint32_t tmem_slot;
-    constexpr int WCOLS = 4 * MAXP;                                  // sum, compensation, of squares, compensation
+    constexpr int WCOLS = 4 * MAXP;                                  // sum, sum of squares
     constexpr uint32_t TCOLS = WCOLS * (NT / 128);
     const int L = ODD ? X : X / 2, HC = X / 2 + 1, XP = a.XP, y = blockIdx.x, t = threadIdx.x, warp = t >> 5;
     float2* const tab = reinterpret_cast<float2*>(pbuf + 2 * L);
@@ -481,7 +483,7 @@ k_pass_c_gen2(const __grid_constant__ BatchArgs a, int X, int Y, const __grid_co
     __syncthreads();
     tmptx::tmem_fence_after_sync();
     const uint32_t tcomp = tmem_slot + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)(WCOLS * (warp >> 2));
-    float mip[MAXP], fs[MAXP], pq[MAXP];
+    float mip[MAXP];
     const size_t rowoff = (size_t)y * X;
     {
         float z[8];
@@ -495,7 +497,6 @@ k_pass_c_gen2(const __grid_constant__ BatchArgs a, int X, int Y, const __grid_co
     for (int j = 0; j < MAXP; j++) {
         const int x = t + NT * j;
         mip[j] = x < X ? a.mip[rowoff + x] : FLT_MAX;   // pixels beyond the row never change
-        fs[j] = pq[j] = 0.f;
     }
     const float2 hmin2 = tmfft::both(a.hist_min), hinv2 = tmfft::both(a.hist_inv_step);
     for (int o = 0; o < a.nb; o += 2) {
@@ -540,67 +541,53 @@ k_pass_c_gen2(const __grid_constant__ BatchArgs a, int X, int Y, const __grid_co
         const float2* zb = reinterpret_cast<const float2*>(pfft_gen<+1, NT, false>(pbuf, pbuf + L, 1, ph, 0, tw));
         const int g = (int)a.gidx0 + o;
 #pragma unroll
-        for (int j = 0; j < MAXP; j++) {
-            const int x = t + NT * j;
-            if (x < X) {
-                const float2 v = zb[ODD ? 2 * x : x];
-                const float m = fmax3(mip[j], v.x, v.y);
-                if (m > mip[j]) a.best[rowoff + x] = v.x == m ? g : g + 1;
-                mip[j] = m;
-                const float2 bv = tmfft::mul2(tmfft::sub2(v, hmin2), hinv2);
-                const int b0 = __float2int_rz(bv.x), b1 = __float2int_rz(bv.y);
-                if ((unsigned)b0 < (unsigned)a.hist_bins) atomicAdd(&shist[b0], 1u);
-                if (two && (unsigned)b1 < (unsigned)a.hist_bins) atomicAdd(&shist[b1], 1u);
-                const float v1 = two ? v.y : 0.f;
-                fs[j] = (fs[j] + v.x) + v1;
-                pq[j] = fmaf(v1, v1, fmaf(v.x, v.x, pq[j]));
-            }
-        }
-        if ((o & 6) == 6 || o + 2 >= a.nb) {
-            // Kahan: the compensation holds what the last addition added beyond its input
+        for (int j0 = 0; j0 < MAXP; j0 += 4) {   // 4 pixels of both sums at a time
+            float sm[8], sq[8];
+            tmptx::tmem_ld8(tcomp + 2 * j0, sm);
+            tmptx::tmem_ld8(tcomp + 2 * MAXP + 2 * j0, sq);
+            tmptx::tmem_wait_ld8x2(sm, sq);
 #pragma unroll
-            for (int sweep = 0; sweep < MAXP / 4; sweep++) {   // 8 pixels of one sum at a time
-                constexpr int HS = MAXP / 8;
-                float* part = (sweep / HS ? pq : fs) + 8 * (sweep % HS);
-                const uint32_t col = tcomp + 2 * MAXP * (sweep / HS) + 8 * (sweep % HS);
-                float sm[8], cm[8];   // sum, compensation
-                tmptx::tmem_ld8(col, sm);
-                tmptx::tmem_ld8(col + MAXP, cm);
-                tmptx::tmem_wait_ld8x2(sm, cm);
-#pragma unroll
-                for (int k = 0; k < 8; k++) {
-                    const float yv = part[k] - cm[k];
-                    const float tv = sm[k] + yv;
-                    cm[k] = (tv - sm[k]) - yv;
-                    sm[k] = tv;
-                    part[k] = 0.f;
+            for (int k = 0; k < 4; k++) {
+                const int j = j0 + k, x = t + NT * j;
+                float2 v = make_float2(0.f, 0.f);   // (beyond the row: added to sums that are never stored)
+                if (x < X) {
+                    v = zb[ODD ? 2 * x : x];
+                    const float m = fmax3(mip[j], v.x, v.y);
+                    if (m > mip[j]) a.best[rowoff + x] = v.x == m ? g : g + 1;
+                    mip[j] = m;
+                    const float2 bv = tmfft::mul2(tmfft::sub2(v, hmin2), hinv2);
+                    const int b0 = __float2int_rz(bv.x), b1 = __float2int_rz(bv.y);
+                    if ((unsigned)b0 < (unsigned)a.hist_bins) atomicAdd(&shist[b0], 1u);
+                    if (two && (unsigned)b1 < (unsigned)a.hist_bins) atomicAdd(&shist[b1], 1u);
+                    if (!two) v.y = 0.f;
                 }
-                tmptx::tmem_st8(col, sm);
-                tmptx::tmem_st8(col + MAXP, cm);
+                double ds = f64_of(sm[2 * k], sm[2 * k + 1]), dq = f64_of(sq[2 * k], sq[2 * k + 1]);
+                const double vx = v.x, vy = v.y;
+                ds = (ds + vx) + vy;
+                dq = fma(vy, vy, fma(vx, vx, dq));
+                f64_to(ds, sm[2 * k], sm[2 * k + 1]);
+                f64_to(dq, sq[2 * k], sq[2 * k + 1]);
             }
-            tmptx::tmem_wait_st();
+            tmptx::tmem_st8(tcomp + 2 * j0, sm);
+            tmptx::tmem_st8(tcomp + 2 * MAXP + 2 * j0, sq);
         }
+        tmptx::tmem_wait_st();
         __syncthreads();   // every output is read before the next pair's rows
     }
 #pragma unroll
-    for (int j0 = 0; j0 < MAXP; j0 += 8) {
+    for (int j0 = 0; j0 < MAXP; j0 += 4) {
+        float sm[8], sq[8];
+        tmptx::tmem_ld8(tcomp + 2 * j0, sm);
+        tmptx::tmem_ld8(tcomp + 2 * MAXP + 2 * j0, sq);
+        tmptx::tmem_wait_ld8x2(sm, sq);
 #pragma unroll
-        for (int k = 0; k < 2; k++) {
-            float sm[8], cm[8];
-            tmptx::tmem_ld8(tcomp + 2 * MAXP * k + j0, sm);
-            tmptx::tmem_ld8(tcomp + 2 * MAXP * k + MAXP + j0, cm);
-            tmptx::tmem_wait_ld8x2(sm, cm);
-            double* const dst = (k ? a.sumsq : a.sum) + rowoff;
-#pragma unroll
-            for (int j = 0; j < 8; j++) {
-                const int x = t + NT * (j0 + j);
-                if (x < X) dst[x] += (double)sm[j] - (double)cm[j];
+        for (int k = 0; k < 4; k++) {
+            const int x = t + NT * (j0 + k);
+            if (x < X) {
+                a.sum[rowoff + x] += f64_of(sm[2 * k], sm[2 * k + 1]);
+                a.sumsq[rowoff + x] += f64_of(sq[2 * k], sq[2 * k + 1]);
+                a.mip[rowoff + x] = mip[j0 + k];
             }
-        }
-#pragma unroll
-        for (int j = j0; j < j0 + 8; j++) {
-            const int x = t + NT * j;
-            if (x < X) a.mip[rowoff + x] = mip[j];
         }
     }
     for (int b = t; b < a.hist_bins; b += NT) {

@@ -23,8 +23,11 @@ def _compensated(x):
     return s.astype(np.float64) - c, q.astype(np.float64) - d
 
 
-# compiled widths below 2048, undivided and divided batches
-@pytest.mark.parametrize("T,X,Y,n", [(32, 256, 256, 6), (32, 256, 256, 33), (64, 512, 512, 40), (64, 1024, 1024, 33)])
+# compiled widths below 2048, undivided and divided batches; run-time sizes of each row pass on pairs
+# (even and odd rows, up to 2048 pixels and above, with and without the tables in shared memory)
+@pytest.mark.parametrize("T,X,Y,n", [(32, 256, 256, 6), (32, 256, 256, 33), (64, 512, 512, 40), (64, 1024, 1024, 33),
+                                     (32, 130, 154, 33), (32, 729, 66, 33), (32, 2700, 66, 24), (32, 2187, 66, 17),
+                                     (32, 3584, 66, 17), (32, 6561, 66, 17), (32, 7280, 66, 17)])
 def test_sums_are_no_less_accurate_than_compensated_ones(T, X, Y, n):
     case = make_case(T=T, X=X, Y=Y, n_particles=1, n_orient=n)
     with core.SearchCore(X, Y, T, histogram_min_scaled=case["hmin"], histogram_step_scaled=case["hstep"]) as sc:
