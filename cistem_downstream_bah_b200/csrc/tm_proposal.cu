@@ -205,7 +205,7 @@ k_conv3x3_wgrad(const float* __restrict__ in, const float* __restrict__ g, float
         for (int k = 0; k < 9; k++) acc[h][k] = make_float2(0.f, 0.f);
     for (int u = blockIdx.y * units; u < min(total, (int)(blockIdx.y + 1) * units); u++) {
         const int n0 = u / bands * NI, y0 = u % bands * RB;
-        bool unbounded = false;   // an input that is infinite or not a number
+        bool unbounded = false;   // an input or a gradient that is infinite or not a number
         // gradients: 4 output channels of a pixel per thread and step
         for (int e = t; e < PX * (OB / 4); e += kThreads) {
             const int p = e % PX, o4 = e / PX * 4;
@@ -215,6 +215,8 @@ k_conv3x3_wgrad(const float* __restrict__ in, const float* __restrict__ g, float
                 const float* gp = g + ((size_t)n * Co + o0 + o4) * (W * W) + y0 * W + r;
 #pragma unroll
                 for (int j = 0; j < 4; j++) v[j] = gp[(size_t)j * (W * W)];
+#pragma unroll
+                for (int j = 0; j < 4; j++) unbounded = unbounded || !(fabsf(v[j]) <= FLT_MAX);
             }
             *reinterpret_cast<float4*>(s_g + p * GP + o4) = make_float4(v[0], v[1], v[2], v[3]);
         }
@@ -234,7 +236,8 @@ k_conv3x3_wgrad(const float* __restrict__ in, const float* __restrict__ g, float
             }
             *reinterpret_cast<float4*>(s_in + q * IB + i4) = make_float4(v[0], v[1], v[2], v[3]);
         }
-        // such an input counts only where its gradient is not zero (the ReLU masks it elsewhere)
+        // such an input counts only where its gradient is not zero (the ReLU masks it elsewhere), such a
+        // gradient only for the taps inside the map
         const bool masked = __syncthreads_or(unbounded);
         // this quarter's 64 pixels, SL of a row at a time
 #pragma unroll 1
@@ -253,6 +256,8 @@ k_conv3x3_wgrad(const float* __restrict__ in, const float* __restrict__ g, float
                 if (masked) {
 #pragma unroll
                     for (int k = 0; k < 9; k++) {
+                        const int yy = y0 + y + k / 3 - 1, xx = x + p + k % 3 - 1;
+                        if (yy < 0 || yy >= W || xx < 0 || xx >= W) continue;
                         const float b = v[k / 3][p + k % 3];
                         if (ga.x != 0.f) acc[0][k].x = fmaf(ga.x, b, acc[0][k].x);
                         if (ga.y != 0.f) acc[0][k].y = fmaf(ga.y, b, acc[0][k].y);
