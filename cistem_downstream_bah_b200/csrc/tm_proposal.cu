@@ -167,7 +167,10 @@ k_conv3x3(const float* __restrict__ in, const __nv_bfloat16* __restrict__ w, con
 // through shared memory; a thread holds the nine sums of 4 output channels x 1
 // input channel over a quarter of them, output channels in pairs: 144 two-wide multiply-adds per 8
 // pixels of a row for 38 loads.  The quarters are added in the block, the blocks with
-// atomics (dW and db are zeroed before the backward pass).  (One block per channel pair read
+// atomics in FP64 (dW and db are zeroed before the backward pass).  A thread adds 16 pixels in one
+// chain and those sums in another: with one chain over all its pixels (256 of 8 x 8 maps, 448 of 16 x 16)
+// and FP32 atomics the error was 1.2 times that of one block per channel pair, with these it is 0.6 to
+// 0.7 of it (third layer, 128 tiles of 32 and 64), for 0.53 instead of 0.50 ms at 128 tiles of 64.  (One block per channel pair read
 // every map from memory once per pair: 0.6-1.95 ms per layer of 128 tiles of 64 x 64; now
 // 0.1-0.2 ms.)
 template <int W>
@@ -180,12 +183,12 @@ struct WGrad {
     static constexpr int E = W + 2;
     static constexpr int IN = NI * (RB + 2) * E * IB;
     static constexpr int SMEM = (PX * GP + IN) * 4;
-    static_assert(IN >= 0 && SMEM >= 3 * 64 * 40 * 4, "the block reduction reuses the staging buffers");
+    static_assert(PX * GP + IN >= 3 * 64 * 40, "the block reduction reuses the staging buffers");
 };
 
 template <int W>
 __global__ void __launch_bounds__(kThreads)
-k_conv3x3_wgrad(const float* __restrict__ in, const float* __restrict__ g, float* dW, float* db, int N, int Ci, int Co, int units) {
+k_conv3x3_wgrad(const float* __restrict__ in, const float* __restrict__ g, double* dW, double* db, int N, int Ci, int Co, int units) {
     using WG = WGrad<W>;
     constexpr int OB = WG::OB, IB = WG::IB, PX = WG::PX, RB = WG::RB, NI = WG::NI, SL = WG::SL, GP = WG::GP, E = WG::E;
     extern __shared__ __align__(16) float wsm[];
@@ -197,12 +200,15 @@ k_conv3x3_wgrad(const float* __restrict__ in, const float* __restrict__ g, float
     const int i = t & 7, og = (t >> 3) & 7, pq = t >> 6;   // input channel, group of 4 output channels, quarter
     constexpr int bands = W / RB;
     const int total = (N + NI - 1) / NI * bands;   // steps
-    float2 acc[2][9];
-    float2 accb[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+    float2 acc[2][10], part[2][10];   // totals and the sums of 16 pixels; tap 9: the bias
+    auto zero = [](float2 (&a)[2][10]) {
 #pragma unroll
-    for (int h = 0; h < 2; h++)
+        for (int h = 0; h < 2; h++)
 #pragma unroll
-        for (int k = 0; k < 9; k++) acc[h][k] = make_float2(0.f, 0.f);
+            for (int k = 0; k < 10; k++) a[h][k] = make_float2(0.f, 0.f);
+    };
+    zero(acc);
+    zero(part);
     for (int u = blockIdx.y * units; u < min(total, (int)(blockIdx.y + 1) * units); u++) {
         const int n0 = u / bands * NI, y0 = u % bands * RB;
         bool unbounded = false;   // an input or a gradient that is infinite or not a number
@@ -259,21 +265,31 @@ k_conv3x3_wgrad(const float* __restrict__ in, const float* __restrict__ g, float
                         const int yy = y0 + y + k / 3 - 1, xx = x + p + k % 3 - 1;
                         if (yy < 0 || yy >= W || xx < 0 || xx >= W) continue;
                         const float b = v[k / 3][p + k % 3];
-                        if (ga.x != 0.f) acc[0][k].x = fmaf(ga.x, b, acc[0][k].x);
-                        if (ga.y != 0.f) acc[0][k].y = fmaf(ga.y, b, acc[0][k].y);
-                        if (gb.x != 0.f) acc[1][k].x = fmaf(gb.x, b, acc[1][k].x);
-                        if (gb.y != 0.f) acc[1][k].y = fmaf(gb.y, b, acc[1][k].y);
+                        if (ga.x != 0.f) part[0][k].x = fmaf(ga.x, b, part[0][k].x);
+                        if (ga.y != 0.f) part[0][k].y = fmaf(ga.y, b, part[0][k].y);
+                        if (gb.x != 0.f) part[1][k].x = fmaf(gb.x, b, part[1][k].x);
+                        if (gb.y != 0.f) part[1][k].y = fmaf(gb.y, b, part[1][k].y);
                     }
                 } else {
 #pragma unroll
                     for (int k = 0; k < 9; k++) {
                         const float2 b = make_float2(v[k / 3][p + k % 3], v[k / 3][p + k % 3]);
-                        acc[0][k] = fma2(ga, b, acc[0][k]);
-                        acc[1][k] = fma2(gb, b, acc[1][k]);
+                        part[0][k] = fma2(ga, b, part[0][k]);
+                        part[1][k] = fma2(gb, b, part[1][k]);
                     }
                 }
-                accb[0].x += ga.x; accb[0].y += ga.y;
-                accb[1].x += gb.x; accb[1].y += gb.y;
+                part[0][9].x += ga.x; part[0][9].y += ga.y;
+                part[1][9].x += gb.x; part[1][9].y += gb.y;
+            }
+            if ((s0 + SL) % 16 == 0) {
+#pragma unroll
+                for (int h = 0; h < 2; h++)
+#pragma unroll
+                    for (int k = 0; k < 10; k++) {
+                        acc[h][k].x += part[h][k].x;
+                        acc[h][k].y += part[h][k].y;
+                    }
+                zero(part);
             }
         }
         __syncthreads();
@@ -282,7 +298,7 @@ k_conv3x3_wgrad(const float* __restrict__ in, const float* __restrict__ g, float
     float* const red = wsm;
     auto value = [&](int e) -> float& {   // e = 10 j + k: output channel j, tap k (9: the bias)
         const int j = e / 10, k = e % 10;
-        float2& a = k < 9 ? acc[j / 2][k] : accb[j / 2];
+        float2& a = acc[j / 2][k];
         return j & 1 ? a.y : a.x;
     };
     if (pq > 0) {
@@ -293,10 +309,10 @@ k_conv3x3_wgrad(const float* __restrict__ in, const float* __restrict__ g, float
     if (pq == 0 && i0 + i < Ci) {
 #pragma unroll
         for (int e = 0; e < 40; e++) {
-            const float v = value(e) + red[e * 64 + t] + red[(40 + e) * 64 + t] + red[(80 + e) * 64 + t];
+            const float v = (value(e) + red[e * 64 + t]) + (red[(40 + e) * 64 + t] + red[(80 + e) * 64 + t]);
             const int o = o0 + 4 * og + e / 10, k = e % 10;
-            if (k < 9) atomicAdd(&dW[((size_t)o * Ci + i0 + i) * 9 + k], v);
-            else if (i0 + i == 0) atomicAdd(&db[o], v);
+            if (k < 9) atomicAdd(&dW[((size_t)o * Ci + i0 + i) * 9 + k], (double)v);
+            else if (i0 + i == 0) atomicAdd(&db[o], (double)v);
         }
     }
 }
@@ -437,6 +453,11 @@ __global__ void k_fc_dgrad(const float* __restrict__ dout, const __nv_bfloat16* 
     dg[e] = s;
 }
 
+__global__ void k_to_f32(const double* __restrict__ src, float* __restrict__ dst, long long n) {
+    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x)
+        dst[e] = (float)src[e];
+}
+
 __global__ void k_to_bf16(const float* __restrict__ src, __nv_bfloat16* __restrict__ dst, long long n) {
     for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x)
         dst[e] = __float2bfloat16_rn(src[e]);
@@ -472,6 +493,7 @@ struct tm_pnet {
     tmp::Layer L[5];
     cudaStream_t stream = nullptr;
     float *p = nullptr, *grad = nullptr, *m = nullptr, *v = nullptr;
+    double* sums = nullptr;   // of the convolutions' gradients, while the blocks add theirs
     __nv_bfloat16* p16 = nullptr;
     int step = 0;
     // activations (max_batch tiles) and their gradients
@@ -573,7 +595,7 @@ int wgrad_launch(tm_pnet* c, const float* in, const float* g, const tmp::Layer& 
     if (shares > total) shares = total;
     const int units = (total + shares - 1) / shares;
     tmp::k_conv3x3_wgrad<W><<<dim3(tiles, (total + units - 1) / units), tmp::kThreads, WG::SMEM, c->stream>>>(
-        in, g, c->grad + l.w, c->grad + l.b, n, l.ci, l.co, units);
+        in, g, c->sums + l.w, c->sums + l.b, n, l.ci, l.co, units);
     PN_CUDA(c, cudaGetLastError());
     return TM_OK;
 }
@@ -596,7 +618,7 @@ int backward(tm_pnet* c, int n, float pos_weight, float dir_weight) {
     const int h1 = c->tile, h2 = h1 / 2, h3 = h1 / 4, h4 = h1 / 8;
     int rc;
     if ((rc = forward(c, n))) return rc;
-    PN_CUDA(c, cudaMemsetAsync(c->grad, 0, sizeof(float) * c->nparam, c->stream));
+    PN_CUDA(c, cudaMemsetAsync(c->sums, 0, sizeof(double) * c->L[4].w, c->stream));
     PN_CUDA(c, cudaMemsetAsync(c->d_loss, 0, sizeof(double), c->stream));
     k_loss<<<(n + 127) / 128, 128, 0, c->stream>>>(c->out, c->lab, c->d_out, c->d_loss, n, pos_weight, dir_weight);
     k_fc_wgrad<<<(kOut * (kC4 + 1) + 127) / 128, 128, 0, c->stream>>>(c->g, c->d_out, c->grad + c->L[4].w,
@@ -622,6 +644,7 @@ int backward(tm_pnet* c, int n, float pos_weight, float dir_weight) {
                                                                                   (long long)n * kC1, h1, h1);
     // layer 1 (no gradient of the input)
     if ((rc = wgrad(c, c->x, c->d_a1, c->L[0], n))) return rc;
+    k_to_f32<<<grid_for(c->L[4].w), 256, 0, c->stream>>>(c->sums, c->grad, c->L[4].w);
     PN_CUDA(c, cudaGetLastError());
     return TM_OK;
 }
@@ -678,6 +701,7 @@ int tm_pnet_create(int device, int in_channels, int tile, int max_batch, tm_pnet
     int rc = TM_OK;
     rc = rc ? rc : palloc(c, &c->p, c->nparam);
     rc = rc ? rc : palloc(c, &c->grad, c->nparam);
+    rc = rc ? rc : palloc(c, &c->sums, c->L[4].w);
     rc = rc ? rc : palloc(c, &c->m, c->nparam);
     rc = rc ? rc : palloc(c, &c->v, c->nparam);
     rc = rc ? rc : palloc(c, &c->p16, c->nparam);
