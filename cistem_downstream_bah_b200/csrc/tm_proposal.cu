@@ -57,37 +57,35 @@ __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
 // forward conv's input channels, i over its output channels), no bias, no ReLU.
 // Every output is one chain of multiply-adds over i, then ky, then kx.
 //
-// Block: a TW x TW tile of output pixels times COB output channels; a thread computes
+// Block: a TW x TW tile of output pixels of NI images times COB output channels; a thread computes
 // PXT pixels of a row x 8 channels, channels in pairs (two multiply-adds per
-// instruction, a pair's weights being adjacent in shared memory): 48 such instructions per
+// instruction, a pair's weights being adjacent in shared memory): with 4 pixels 48 such instructions per
 // input channel and kernel row for 8 shared-memory loads.  (One pixel x 8 channels with
 // 9 loads per 8 multiply-adds: the shared-memory pipe bound it at a sixth of the FP32 rate, 200-417
-// us for the layers of 128 tiles of 64 x 64; 85-172 now.)  Input channels go through
+// us for the layers of 128 tiles of 64 x 64; 85-168 now.)  Input channels go through
 // shared memory CIB at a time with their halo.
-template <int TW>
+template <int TW_, int PXT_, int CG_, int NI_>
 struct ConvTile {
+    static constexpr int TW = TW_, PXT = PXT_, CG = CG_, NI = NI_;
     static constexpr int CIB = 8, COT = 8;
-    static constexpr int PXT = TW < 4 ? TW : 4;
-    static constexpr int PG = TW * TW / PXT;                            // pixel groups
-    static constexpr int CG = PG >= 64 ? 4 : PG >= 16 ? 8 : 16;         // channel groups
-    static constexpr int COB = CG * COT, NT = PG * CG;
+    static constexpr int PG = TW * TW / PXT;                            // pixel groups of an image
+    static constexpr int COB = CG * COT, NT = NI * PG * CG;
     static constexpr int PITCH = (TW + 2 + 3) / 4 * 4;                  // row pitch of the input tile, 16-byte aligned
 };
 
-template <bool FLIP, int TW>
-__global__ void __launch_bounds__(ConvTile<TW>::NT)
+template <bool FLIP, class CT>
+__global__ void __launch_bounds__(CT::NT)
 k_conv3x3(const float* __restrict__ in, const __nv_bfloat16* __restrict__ w, const float* __restrict__ bias,
-          float* __restrict__ out, int Ci, int Co, int H, int relu) {
-    using CT = ConvTile<TW>;
-    constexpr int CIB = CT::CIB, PXT = CT::PXT, COB = CT::COB, NT = CT::NT, PITCH = CT::PITCH, E = TW + 2;
-    __shared__ __align__(16) float s_in[CIB][E][PITCH];
+          float* __restrict__ out, int N, int Ci, int Co, int H, int relu) {
+    constexpr int TW = CT::TW, CIB = CT::CIB, PXT = CT::PXT, COB = CT::COB, NT = CT::NT, NI = CT::NI, PITCH = CT::PITCH, E = TW + 2;
+    __shared__ __align__(16) float s_in[NI][CIB][E][PITCH];
     __shared__ __align__(16) float s_w[CIB][9][COB];
     const int tiles_x = H / TW;
     const int ty0 = (blockIdx.x / tiles_x) * TW, tx0 = (blockIdx.x % tiles_x) * TW;
     const int co0 = blockIdx.y * COB;
-    const int n = blockIdx.z;
     const int t = threadIdx.x;
-    const int pg = t % CT::PG, cg = t / CT::PG;
+    const int pg = t % CT::PG, im = t / CT::PG % NI, cg = t / (CT::PG * NI);
+    const int n0 = blockIdx.z * NI, n = n0 + im;
     const int py = pg / (TW / PXT), px = pg % (TW / PXT) * PXT;
     float2 acc[PXT][4];
 #pragma unroll
@@ -95,14 +93,14 @@ k_conv3x3(const float* __restrict__ in, const __nv_bfloat16* __restrict__ w, con
 #pragma unroll
         for (int j = 0; j < 4; j++) acc[p][j] = make_float2(0.f, 0.f);
     for (int ci0 = 0; ci0 < Ci; ci0 += CIB) {
-        // input tile with halo
-        for (int e = t; e < CIB * E * E; e += NT) {
-            const int c = e / (E * E), r = e % (E * E);
+        // input tiles with halo
+        for (int e = t; e < NI * CIB * E * E; e += NT) {
+            const int c = e / (E * E), r = e % (E * E);   // image and channel
             const int yy = ty0 + r / E - 1, xx = tx0 + r % E - 1;
-            const int ci = ci0 + c;
+            const int nn = n0 + c / CIB, ci = ci0 + c % CIB;
             float v = 0.0f;
-            if (ci < Ci && yy >= 0 && yy < H && xx >= 0 && xx < H) v = in[(((size_t)n * Ci + ci) * H + yy) * H + xx];
-            s_in[c][r / E][r % E] = v;
+            if ((NI == 1 || nn < N) && ci < Ci && yy >= 0 && yy < H && xx >= 0 && xx < H) v = in[(((size_t)nn * Ci + ci) * H + yy) * H + xx];
+            s_in[c / CIB][c % CIB][r / E][r % E] = v;
         }
         // weights of COB output channels x CIB input channels, channel fastest
         for (int e = t; e < COB * CIB * 9; e += NT) {
@@ -121,7 +119,7 @@ k_conv3x3(const float* __restrict__ in, const __nv_bfloat16* __restrict__ w, con
         for (int c = 0; c < CIB; c++) {
 #pragma unroll
             for (int ky = 0; ky < 3; ky++) {
-                const float* row = &s_in[c][py + ky][px];
+                const float* row = &s_in[im][c][py + ky][px];
                 float v[PXT + 2];
                 if constexpr (PXT == 4) {
                     const float4 a = *reinterpret_cast<const float4*>(row);
@@ -146,6 +144,7 @@ k_conv3x3(const float* __restrict__ in, const __nv_bfloat16* __restrict__ w, con
         }
         __syncthreads();
     }
+    if (NI > 1 && n >= N) return;
     const int y = ty0 + py, x = tx0 + px;
 #pragma unroll
     for (int j = 0; j < CT::COT; j++) {
@@ -541,27 +540,40 @@ int grid_for(long long n) {
     return (int)(b < 148LL * 16 ? (b > 0 ? b : 1) : 148LL * 16);
 }
 
-template <bool FLIP, int TW>
+// grid (spatial tiles, output-channel groups, groups of images)
+template <bool FLIP, class CT>
 void conv_launch(tm_pnet* c, const float* in, const float* bias, float* out, const tmp::Layer& l, int n, int relu) {
-    using CT = tmp::ConvTile<TW>;
     const int H = l.h, ci = FLIP ? l.co : l.ci, co = FLIP ? l.ci : l.co;
-    const dim3 grid((H / TW) * (H / TW), (co + CT::COB - 1) / CT::COB, n);
-    tmp::k_conv3x3<FLIP, TW><<<grid, CT::NT, 0, c->stream>>>(in, c->p16 + l.w, bias, out, ci, co, H, relu);
+    const dim3 grid((H / CT::TW) * (H / CT::TW), (co + CT::COB - 1) / CT::COB, (n + CT::NI - 1) / CT::NI);
+    tmp::k_conv3x3<FLIP, CT><<<grid, CT::NT, 0, c->stream>>>(in, c->p16 + l.w, bias, out, n, ci, co, H, relu);
 }
 
-// launch of one conv: grid (spatial tiles, output-channel groups, images)
+// The form with one pixel per thread, fewer channels per block and so more blocks while these are
+// at most one per SM (then a layer's time is that of one block, whatever their number), else the one with
+// the most multiply-adds per load.  128 -> 128 channels, us at 2 / 32 / 128 / 1024 images,
+// first form and second: 2 x 2 maps 61 / 69 / 69 / 153 and 66 / 85 / 85 / 109, 4 x 4
+// 71 / 72 / 93 / 499 and 89 / 105 / 105 / 221; 2 / 32 / 64 / 128 images: 8 x 8 75 / 77 / 116 / 207 and
+// 109 / 110 / 110 / 146, 16 x 16 (64 -> 128) 40 / 79 / 132 / 249 and 56 / 58 / 85 / 163.
+template <bool FLIP, class FEW, class MANY>
+void conv_few_or_many(tm_pnet* c, const float* in, const float* bias, float* out, const tmp::Layer& l, int n, int relu) {
+    const int co = FLIP ? l.ci : l.co, tiles = (l.h / FEW::TW) * (l.h / FEW::TW);
+    const long long blocks = (long long)tiles * ((co + FEW::COB - 1) / FEW::COB) * ((n + FEW::NI - 1) / FEW::NI);
+    if (blocks <= c->nsm) conv_launch<FLIP, FEW>(c, in, bias, out, l, n, relu);
+    else conv_launch<FLIP, MANY>(c, in, bias, out, l, n, relu);
+}
+
+template <bool FLIP>
+void conv_dispatch(tm_pnet* c, const float* in, const float* bias, float* out, const tmp::Layer& l, int n, int relu) {
+    using tmp::ConvTile;
+    if (l.h >= 16) conv_few_or_many<FLIP, ConvTile<16, 1, 1, 1>, ConvTile<16, 4, 4, 1>>(c, in, bias, out, l, n, relu);
+    else if (l.h == 8) conv_few_or_many<FLIP, ConvTile<8, 1, 4, 1>, ConvTile<8, 4, 8, 1>>(c, in, bias, out, l, n, relu);
+    else if (l.h == 4) conv_few_or_many<FLIP, ConvTile<4, 1, 4, 2>, ConvTile<4, 4, 4, 8>>(c, in, bias, out, l, n, relu);
+    else conv_few_or_many<FLIP, ConvTile<2, 1, 2, 16>, ConvTile<2, 2, 2, 32>>(c, in, bias, out, l, n, relu);
+}
+
 int conv(tm_pnet* c, bool flip, const float* in, const float* bias, float* out, const tmp::Layer& l, int n, int relu) {
-    if (flip) {
-        if (l.h >= 16) conv_launch<true, 16>(c, in, nullptr, out, l, n, 0);
-        else if (l.h == 8) conv_launch<true, 8>(c, in, nullptr, out, l, n, 0);
-        else if (l.h == 4) conv_launch<true, 4>(c, in, nullptr, out, l, n, 0);
-        else conv_launch<true, 2>(c, in, nullptr, out, l, n, 0);
-    } else {
-        if (l.h >= 16) conv_launch<false, 16>(c, in, bias, out, l, n, relu);
-        else if (l.h == 8) conv_launch<false, 8>(c, in, bias, out, l, n, relu);
-        else if (l.h == 4) conv_launch<false, 4>(c, in, bias, out, l, n, relu);
-        else conv_launch<false, 2>(c, in, bias, out, l, n, relu);
-    }
+    if (flip) conv_dispatch<true>(c, in, nullptr, out, l, n, 0);
+    else conv_dispatch<false>(c, in, bias, out, l, n, relu);
     PN_CUDA(c, cudaGetLastError());
     return TM_OK;
 }
