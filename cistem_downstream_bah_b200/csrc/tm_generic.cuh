@@ -440,9 +440,10 @@ __global__ void __launch_bounds__(kGenNT) k_pass_b_gen2(const __grid_constant__ 
 // inverse of the Hermitian extension, the imaginary part of the DC term ignored as FFTW's
 // c2r does.  The best orientation goes to memory when a pixel's maximum changes.  256
 // threads where two blocks fit an SM (up to 3,072 pixels), else 512.  Shared memory: 2 x L pairs
-// | the twiddle table (TAB) | the next pair's rows of C (TAB) | histogram.
+// | the twiddle table (TAB) | the next pair's rows of C (TAB) | histogram, TMEM slot (no static shared memory:
+// the limit is on both together).
 __host__ __device__ constexpr size_t gen_pass_c_smem(int X, int XP, int bins, bool tab) {
-    return sizeof(float4) * (X % 2 ? 2 * X : X) + (tab ? sizeof(float2) * (X + X % 2 + 2 * XP) : 0) + 4 * (size_t)bins;
+    return sizeof(float4) * (X % 2 ? 2 * X : X) + (tab ? sizeof(float2) * (X + X % 2 + 2 * XP) : 0) + 4 * ((size_t)bins + 1);
 }
 // pairs of rows fit shared memory (else k_pass_c_gen)
 inline bool gen_pass_c_pairs(int X, int XP, int bins) { return gen_pass_c_smem(X, XP, bins, false) <= 232448; }
@@ -451,15 +452,15 @@ template <bool ODD, int MAXP, int NT, bool TAB>
 __global__ void __launch_bounds__(NT, NT == 512 ? 1 : 2)
 k_pass_c_gen2(const __grid_constant__ BatchArgs a, int X, int Y, const __grid_constant__ GenPlan ph) {
     extern __shared__ __align__(16) float4 pbuf[];   // 2 x L, L = X/2 or X
-    __shared__ uint32_t tmem_slot;
     constexpr int WCOLS = 4 * MAXP;                                  // sum, sum of squares
     constexpr uint32_t TCOLS = WCOLS * (NT / 128);
     const int L = ODD ? X : X / 2, HC = X / 2 + 1, XP = a.XP, y = blockIdx.x, t = threadIdx.x, warp = t >> 5;
     float2* const tab = reinterpret_cast<float2*>(pbuf + 2 * L);
     float2* const rows = tab + X + X % 2;                            // two rows of XP
     unsigned int* const shist = reinterpret_cast<unsigned int*>(TAB ? rows + 2 * XP : tab);
+    uint32_t* const tmem_slot = shist + a.hist_bins;
     if (warp == 0) {
-        tmptx::tmem_alloc(&tmem_slot, TCOLS);
+        tmptx::tmem_alloc(tmem_slot, TCOLS);
         tmptx::tmem_relinquish();
     }
     for (int b = t; b < a.hist_bins; b += NT) shist[b] = 0u;
@@ -482,7 +483,7 @@ k_pass_c_gen2(const __grid_constant__ BatchArgs a, int X, int Y, const __grid_co
     tmptx::tmem_fence_before_sync();
     __syncthreads();
     tmptx::tmem_fence_after_sync();
-    const uint32_t tcomp = tmem_slot + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)(WCOLS * (warp >> 2));
+    const uint32_t tcomp = *tmem_slot + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)(WCOLS * (warp >> 2));
     float mip[MAXP];
     const size_t rowoff = (size_t)y * X;
     {
@@ -597,7 +598,7 @@ k_pass_c_gen2(const __grid_constant__ BatchArgs a, int X, int Y, const __grid_co
     tmptx::tmem_fence_before_sync();
     __syncthreads();
     tmptx::tmem_fence_after_sync();
-    if (warp == 0) tmptx::tmem_dealloc(tmem_slot, TCOLS);
+    if (warp == 0) tmptx::tmem_dealloc(*tmem_slot, TCOLS);
 }
 
 // the row pass for a width X: kernel, threads and shared memory
