@@ -29,6 +29,7 @@
 #include <type_traits>
 
 #include "tm_fft.cuh"
+#include "tm_generic_forms.h"
 #include "tm_whiten.cuh"
 
 namespace tmk {
@@ -384,11 +385,8 @@ __global__ void __launch_bounds__(256) k_pass_a_gen2(const __grid_constant__ Bat
 }
 
 // k_pass_b_gen2: block per (LP pairs of adjacent columns, `ob` orientations in turn).
-// Shared memory: 2 x LP x Y pairs | the twiddle table (TAB) | the next orientation's rows of A.
-__host__ __device__ constexpr size_t gen_pass_b_smem(int LP, int T, int Y, bool tab) {
-    return sizeof(float4) * 2 * LP * Y + (tab ? sizeof(float2) * (Y + Y % 2) : 0) + sizeof(float4) * LP * T;
-}
-template <int LP, bool TAB>
+// Shared memory: gen_pass_b_smem.
+template <int LP, bool TAB, bool STAGED>
 __global__ void __launch_bounds__(kGenNT) k_pass_b_gen2(const __grid_constant__ BatchArgs a, int T, int Y, int ob, const __grid_constant__ GenPlan py) {
     extern __shared__ __align__(16) float4 pbuf[];   // pair c of a buffer at c * Y
     float4* const tmp = pbuf + LP * Y;
@@ -409,16 +407,19 @@ __global__ void __launch_bounds__(kGenNT) k_pass_b_gen2(const __grid_constant__ 
         }
         tmptx::cp_async_commit();
     };
-    issue_rows(o0);
+    if constexpr (STAGED) issue_rows(o0);
     for (int o = o0; o < o1; o++) {
-        tmptx::cp_async_wait<0>();
+        if constexpr (STAGED) tmptx::cp_async_wait<0>();
         __syncthreads();   // the rows (and the table); the previous orientation's output is stored
         const int s0 = pfill_pruned<kGenNT>(pbuf, LP, T, py, [&](int c, int n) {
-            const float4 v = astage[n * LP + c];
+            const float4 v = STAGED ? astage[n * LP + c]
+                                    : __ldg(reinterpret_cast<const float4*>(a.A + ((size_t)o * T + n) * XP + kx0 + 2 * c));
             return make_float4(v.x, v.z, v.y, v.w);
         });
         __syncthreads();
-        if (o + 1 < o1) issue_rows(o + 1);
+        if constexpr (STAGED) {
+            if (o + 1 < o1) issue_rows(o + 1);
+        }
         float4* f = pfft_gen<-1, kGenNT, false>(pbuf, tmp, LP, py, s0, tw);
         const float4* z = pfft_gen<+1, kGenNT, true>(f, f == pbuf ? tmp : pbuf, LP, py, 0, tw,
                                                      reinterpret_cast<const float4*>(a.Ip + kx0), XP / 2);
@@ -446,7 +447,7 @@ __host__ __device__ constexpr size_t gen_pass_c_smem(int X, int XP, int bins, bo
     return sizeof(float4) * (X % 2 ? 2 * X : X) + (tab ? sizeof(float2) * (X + X % 2 + 2 * XP) : 0) + 4 * ((size_t)bins + 1);
 }
 // pairs of rows fit shared memory (else k_pass_c_gen)
-inline bool gen_pass_c_pairs(int X, int XP, int bins) { return gen_pass_c_smem(X, XP, bins, false) <= 232448; }
+inline bool gen_pass_c_pairs(int X, int XP, int bins) { return gen_pass_c_smem(X, XP, bins, false) <= kBlockSharedLimit; }
 
 template <bool ODD, int MAXP, int NT, bool TAB>
 __global__ void __launch_bounds__(NT, NT == 512 ? 1 : 2)
@@ -610,7 +611,7 @@ struct GenRowPass {
 template <bool ODD>
 inline GenRowPass gen_row_pass_pairs(int X, int XP, int bins) {
     const size_t full = gen_pass_c_smem(X, XP, bins, true);
-    const bool tab = full <= 232448;
+    const bool tab = full <= kBlockSharedLimit;
     const size_t smem = tab ? full : gen_pass_c_smem(X, XP, bins, false);
     if (X <= 2048 && full <= 113 * 1024) return {k_pass_c_gen2<ODD, 8, 256, true>, 256, full};
     if (X <= 4096 && full <= 113 * 1024) return {k_pass_c_gen2<ODD, 16, 256, true>, 256, full};
@@ -628,15 +629,12 @@ struct GenColPass {
     size_t smem;
 };
 inline GenColPass gen_col_pass(int T, int Y) {
-    for (int lp = 2; lp >= 1; lp--)
-        for (int tab = 1; tab >= 0; tab--) {
-            const size_t smem = gen_pass_b_smem(lp, T, Y, tab);
-            if (smem > 232448) continue;
-            return {lp == 2 ? (tab ? k_pass_b_gen2<2, true> : k_pass_b_gen2<2, false>)
-                            : (tab ? k_pass_b_gen2<1, true> : k_pass_b_gen2<1, false>),
-                    2 * lp, smem};
-        }
-    return {k_pass_b_gen, 1, sizeof(float2) * 2 * Y};
+    const GenColForm f = gen_col_form(T, Y);
+    auto* kernel = f.pairs == 2 ? (f.tab ? k_pass_b_gen2<2, true, true> : k_pass_b_gen2<2, false, true>)
+                   : f.pairs == 1 ? (f.tab ? k_pass_b_gen2<1, true, true>
+                                     : f.staged ? k_pass_b_gen2<1, false, true> : k_pass_b_gen2<1, false, false>)
+                                  : k_pass_b_gen;
+    return {kernel, f.columns(), f.smem};
 }
 // orientations per block: up to 8, which share the table and overlap the loads, as long as there are two
 // blocks per SM (352 x 1331, 9 orientations: 0.13 ms with 8, 0.06 one by one)
