@@ -1100,14 +1100,22 @@ struct PassC {
     static constexpr uint32_t TMEM_COLS = WCOLS * ((NT / 32 + 3) / 4);   // warps of a lane quadrant side by side
     static_assert(PL::radix(0) == 8 && PL::radix(1) == 8 && (PL::stages == 3 || PL::stages == 4) && G <= 32, "pass C widths");
     // blocks that share a group of rows of an image of height Y: as many as are resident together
-    static int parts(int Y, int nsm) {
+    static int parts(int Y, int resident) {
         int n = 1;
-        while (n < kPassCParts && Y / ROWS * 2 * n <= MIN_BLOCKS * nsm) n *= 2;
+        while (n < kPassCParts && Y / ROWS * 2 * n <= resident) n *= 2;
         return n;
     }
     // dynamic shared memory for a row pitch XP and `bins` histogram bins (one word for values outside)
     static size_t smem_bytes(int XP, int bins) {
         return 128 + sizeof(float2) * (size_t)ROWS * 2 * c_row_len(XP) + sizeof(float4) * 2 * (size_t)ROWS * EXL + 4 * ((size_t)bins + 1);
+    }
+    // blocks resident per SM (228 KB, 1 KB of it the system's per block): MIN_BLOCKS up to about 860 bins,
+    // one fewer above to 2048 pixels, where a grid of MIN_BLOCKS leaves the last blocks to a second wave
+    // (with 1024 bins: 2048 x 2916, 128 orientations 1.35 ms, 1.18 so; 512 x 512, 512 orientations 0.377 in
+    // four parts, 0.369 in the two that are resident)
+    static int resident(int XP, int bins) {
+        const int n = (int)(233472 / (smem_bytes(XP, bins) + 1024));
+        return n < MIN_BLOCKS ? n : MIN_BLOCKS;
     }
 };
 
@@ -1649,7 +1657,7 @@ struct Launch {
     static constexpr bool RG = (T == 256 && Y == 4096);
     // images whose row pass divides its batches (PassC::parts)
     static constexpr bool DIVIDES = 2 * (Y / PC::ROWS) <= PC::MIN_BLOCKS * 160;
-    static int pass_c_parts(int nsm) { return DIVIDES ? PC::parts(Y, nsm) : 1; }
+    static int pass_c_parts(int nsm) { return DIVIDES ? PC::parts(Y, PC::MIN_BLOCKS * nsm) : 1; }   // most
     static cudaError_t configure_b() {
         cudaError_t e = configure_cols(k_pass_b<T, Y>, PB::SMEM);
         if (RG && e == cudaSuccess)
@@ -1681,11 +1689,11 @@ struct Launch {
             k_pass_b<T, Y><<<PB::BPS * nsm, PB::NT, PB::SMEM, s>>>(a, ngroups);
     }
     static void pass_c(BatchArgs& a, const CMaps& cmaps, cudaStream_t s, int nsm) {
-        const int nblocks = Y / PC::ROWS, resident = PC::MIN_BLOCKS * nsm;
+        const int nblocks = Y / PC::ROWS, resident = PC::resident(a.XP, a.hist_bins) * nsm;
         const size_t smem = PC::smem_bytes(a.XP, a.hist_bins);
         if constexpr (DIVIDES) {
             // at least two pairs of orientations for each part
-            int parts = a.best_parts ? PC::parts(Y, nsm) : 1;
+            int parts = a.best_parts ? PC::parts(Y, resident) : 1;
             while (parts > 1 && a.nb < 4 * parts) parts /= 2;
             if (parts > 1) {
                 cudaLaunchAttribute cluster;
