@@ -527,7 +527,7 @@ k_pass_b(BatchArgs a, int ngroups) {
     using tmfft::Pair;
     constexpr int W = PB::W, WP = PB::WP, MY = PB::MY, PT = PB::PT, NT = PB::NT, V = PB::V, P = PB::P, L = PB::L;
     const int XP = a.XP;
-    extern __shared__ __align__(16) unsigned char smem_b[];
+    extern __shared__ __align__(128) unsigned char smem_b[];
     float4* exch = reinterpret_cast<float4*>(smem_b);
     float4* abuf = reinterpret_cast<float4*>(smem_b + PB::EXCH);
     float4* w01 = reinterpret_cast<float4*>(smem_b + PB::EXCH + PB::ABUFS * PB::ASZ);
@@ -1200,7 +1200,7 @@ k_pass_c(BatchArgs a, const __grid_constant__ CUtensorMap cmap, int Y, int parts
     using PC = PassC<X>;
     using PL = typename PC::PL;
     using TW = PassCTw<X>;
-    constexpr int P = PC::P, G = PC::G, S = PC::S, NT = PC::NT, ROWS = PC::ROWS, EXL = PC::EXL, H = PC::H;
+    constexpr int P = PC::P, G = PC::G, S = PC::S, NT = PC::NT, ROWS = PC::ROWS, EXL = PC::EXL;
     constexpr uint32_t kWaitLimit = 1u << 24;
     const int LR = c_row_len(a.XP);   // float2 of a row in shared memory
     // dynamic shared memory: mbarrier, TMEM slot | row pair | exchange 0 | exchange 1 | histogram

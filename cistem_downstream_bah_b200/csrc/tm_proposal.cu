@@ -32,22 +32,14 @@
 #include <vector>
 
 #include "../../include/tm_b200.h"
+#include "tm_fft.cuh"
 
 namespace tmp {
 
 constexpr int kC1 = 32, kC2 = 64, kC3 = 128, kC4 = 128, kOut = 4;
 constexpr int kThreads = 256;
 
-// ----------------------------------------------------------------------------------------------
-// Two FP32 multiply-adds in one issue slot (sm_100's fma.f32x2, each half rounded as fmaf)
-__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
-    float2 r;
-    asm("{\n\t.reg .b64 p, q, s, t;\n\tmov.b64 p, {%2, %3};\n\tmov.b64 q, {%4, %5};\n\tmov.b64 s, {%6, %7};\n\t"
-        "fma.rn.f32x2 t, p, q, s;\n\tmov.b64 {%0, %1}, t;\n\t}"
-        : "=f"(r.x), "=f"(r.y)
-        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
-    return r;
-}
+using tmfft::fma2;
 
 // ----------------------------------------------------------------------------------------------
 // 3x3 convolution, zero padding 1, NCHW.  out[n][o][y][x] = b[o] + sum_i sum_k
