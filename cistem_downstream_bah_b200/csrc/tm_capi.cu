@@ -976,8 +976,7 @@ int tm_create(const tm_dims* dims, tm_ctx** out) {
     c->Y = dims->image_y;
     c->T = dims->template_size;
     c->TP = c->T / 2 + 1;
-    c->B = dims->orientation_batch > 0 ? dims->orientation_batch : 32;
-    c->Bcap = dims->orientation_batch > 0 ? dims->orientation_batch : 128;   // 0 = automatic: room to tune up to 128
+    c->B = c->Bcap = dims->orientation_batch > 0 ? dims->orientation_batch : 128;   // 0 = automatic
     if (dims->histogram_bins <= 0 || dims->histogram_bins > 1024 || !(dims->histogram_step_scaled > 0)) {
         *out = c;
         return set_err(c, TM_ERR_INVALID, "histogram_bins must be 1..1024 and the step positive");

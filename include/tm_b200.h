@@ -52,13 +52,14 @@ typedef struct tm_dims {
     int histogram_bins;            /* 512 in the reference */
     double histogram_min_scaled;   /* histogram_min / sqrt(X*Y) */
     double histogram_step_scaled;  /* histogram_step / sqrt(X*Y) */
-    int orientation_batch;         /* orientations per device pass; 0 = automatic (32 until
-                                      tm_autotune_batch picks 16, 32, 64 or 128) */
+    int orientation_batch;         /* orientations per device pass; 0 = automatic: 128, or 64 or 32 where
+                                      128 correlation spectra do not fit a quarter of the free device
+                                      memory at tm_create, until tm_autotune_batch picks a batch */
     int device;                    /* CUDA device ordinal */
 } tm_dims;
 
-/* Called after each device pass with the number of orientations finished in
- * the current plane; a non-zero return cancels the plane (TM_ERR_CANCELLED). */
+/* Called after each device pass (orientation_batch orientations) with the number
+ * of orientations finished in the current plane; a non-zero return cancels the plane (TM_ERR_CANCELLED). */
 typedef int (*tm_progress_fn)(long long orientations_done, long long orientations_total, void *user);
 
 /* Replaces TemplateMatchingCore::Init's device set-up (TemplateMatchingCore.cu:49-138):
