@@ -22,8 +22,10 @@
 //   k_w_rows_gen,  the whitening's row r2c and column FFT (with the quadrant
 //   k_w_cols_gen   swap and zeroed central pixel)
 //
-// The arithmetic is the compiled path's (FP32, the same packing, twiddle
-// tables and epilogue); only the FFT organisation differs.  Lines up to
+// The arithmetic is the compiled path's (FP32, the same packing and twiddle
+// tables; FP64 sums of every value as at compiled widths below 2048, but for the
+// longest odd rows, whose sums are FP32, compensated at each value); only the FFT
+// organisation differs.  Lines up to
 // kGenMaxLen = 8192 points.
 #pragma once
 #include <type_traits>

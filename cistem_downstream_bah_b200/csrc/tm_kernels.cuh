@@ -462,8 +462,8 @@ static_assert(sizeof(ColSchedule) <= 48, "the schedule sits in the last 48 bytes
 // What bounds it: the FP32 pipe (44 % busy at 256 x 3888; one item's loads, butterflies and stores take turns
 // at the block's barriers), then its writes of C.  One column per thread -> this, 32
 // orientations of 4096 columns: 256 x 3888 1.52 -> 1.46 ms, 384 x 5832 3.36 -> 2.39; 33 of 2048 columns: 256 x 2916 0.70
-// -> 0.53, 256 x 2592 0.85 -> 0.70; 96 of 1024: 64 x 1024 0.21 -> 0.17; 96 of 512: 256 x 512 0.073 -> 0.059; below 0.02 ms
-// (32 x 256) a launch gains nothing.  (At 5832, both pairs of a thread one after the other, without spills but
+// -> 0.53, 256 x 2592 0.85 -> 0.70; 96 of 1024: 64 x 1024 0.21 -> 0.17; 96 of 512: 256 x 512 0.073 -> 0.059; the
+// smallest lose a little (96 of 256: 32 x 256 0.023 -> 0.025).  (At 5832, both pairs of a thread one after the other, without spills but
 // with 11 warps: 2.73 ms.)
 // The forward transform along y is pruned: MY = Y/L twiddled L-point transforms
 // of the T rows of A zero-padded to L (L = T for power-of-two heights).
