@@ -31,6 +31,7 @@
 #include <cuda.h>
 #include <cuda_fp16.h>
 #include <float.h>
+#include <type_traits>
 #include "tm_fft.cuh"
 #include "tm_ptx.cuh"
 
@@ -1091,8 +1092,8 @@ struct PassC {
     // Widths whose sums take every value by itself: plain FP32 sums over 8 orientations have 2.7 times the
     // error of sums compensated at each (128 orientations of unit noise: 6.2e-7 against 2.3e-7,
     // emulated), FP64 has none to speak of.  The conversions share their unit with those of the histogram: 512
-    // orientations at 1024 x 1024 0.81 ms with plain sums, 0.90 so (0.97 with two-term FP32 sums of
-    // each value); 512 x 512 0.287 both; 256 x 256 0.143 and 0.148
+    // orientations at 1024 x 1024 0.81 ms with plain sums, 0.87 so (0.97 with two-term FP32 sums of
+    // each value); 512 x 512 0.287 and 0.278; 256 x 256 0.143 both
     static constexpr bool EXACT = X < 2048;
     // 512 threads per SM at 128 registers: every block has its 128 TMEM columns per warp
     static constexpr int MIN_BLOCKS = 512 / NT;
@@ -1390,65 +1391,66 @@ k_pass_c(BatchArgs a, const __grid_constant__ CUtensorMap cmap, int Y, int parts
             const unsigned int bin = (unsigned int)__float2int_rz(b);
             atomicAdd(&shist[bin < nbins ? bin : nbins], 1u);
         };
-        auto bins = [&](int r) {
-            const float2 p = val(r);
-            if (two) {
-                const float2 b = tmfft::fma2(p, hinv2, hoff2);
-                count(b.x);
-                count(b.y);
+        // the sums and the histogram, compiled for a pair and for the single last one of an odd batch (a branch at
+        // each pixel cost the EXACT form 4 %)
+        auto add = [&](auto pair) {
+            constexpr bool both = decltype(pair)::value;
+            auto bins = [&](int r) {
+                const float2 p = val(r);
+                if constexpr (both) {
+                    const float2 b = tmfft::fma2(p, hinv2, hoff2);
+                    count(b.x);
+                    count(b.y);
+                } else {
+                    count(fmaf(p.x, a.hist_inv_step, hoff));
+                }
+            };
+            if constexpr (PC::EXACT) {
+                // FP64 sums of pixel r in columns 2 r (sum) and 32 + 2 r (sum of squares), 4 pixels at a
+                // time, whose bins are counted while the sums arrive
+#pragma unroll
+                for (int h = 0; h < 4; h++) {
+                    float sm[8], sq[8];
+                    tmptx::tmem_ld8(tcomp + 8 * h, sm);
+                    tmptx::tmem_ld8(tcomp + 32 + 8 * h, sq);
+#pragma unroll
+                    for (int k = 0; k < 4; k++) bins(4 * h + k);
+                    tmptx::tmem_wait_ld8x2(sm, sq);
+#pragma unroll
+                    for (int k = 0; k < 4; k++) {
+                        const float2 p = val(4 * h + k);
+                        double ds = f64_of(sm[2 * k], sm[2 * k + 1]), dq = f64_of(sq[2 * k], sq[2 * k + 1]);
+                        const double x = p.x;
+                        ds += x;
+                        dq = fma(x, x, dq);
+                        if constexpr (both) {
+                            const double y = p.y;
+                            ds += y;
+                            dq = fma(y, y, dq);
+                        }
+                        f64_to(ds, sm[2 * k], sm[2 * k + 1]);
+                        f64_to(dq, sq[2 * k], sq[2 * k + 1]);
+                    }
+                    tmptx::tmem_st8(tcomp + 8 * h, sm);
+                    tmptx::tmem_st8(tcomp + 32 + 8 * h, sq);
+                }
+                tmptx::tmem_wait_st();
             } else {
-                count(fmaf(p.x, a.hist_inv_step, hoff));
+#pragma unroll
+                for (int r = 0; r < 16; r++) {
+                    const float2 p = val(r);
+                    fs[r] += p.x;
+                    pq[r] = fmaf(p.x, p.x, pq[r]);
+                    if constexpr (both) {
+                        fs[r] += p.y;
+                        pq[r] = fmaf(p.y, p.y, pq[r]);
+                    }
+                    bins(r);
+                }
             }
         };
-        if constexpr (PC::EXACT) {
-            // FP64 sums of pixel r in columns 2 r (sum) and 32 + 2 r (sum of squares), 4 pixels at a
-            // time, whose bins are counted while the sums arrive
-#pragma unroll
-            for (int h = 0; h < 4; h++) {
-                float sm[8], sq[8];
-                tmptx::tmem_ld8(tcomp + 8 * h, sm);
-                tmptx::tmem_ld8(tcomp + 32 + 8 * h, sq);
-#pragma unroll
-                for (int k = 0; k < 4; k++) bins(4 * h + k);
-                tmptx::tmem_wait_ld8x2(sm, sq);
-#pragma unroll
-                for (int k = 0; k < 4; k++) {
-                    const float2 p = val(4 * h + k);
-                    double ds = f64_of(sm[2 * k], sm[2 * k + 1]), dq = f64_of(sq[2 * k], sq[2 * k + 1]);
-                    const double x = p.x;
-                    ds += x;
-                    dq = fma(x, x, dq);
-                    if (two) {
-                        const double y = p.y;
-                        ds += y;
-                        dq = fma(y, y, dq);
-                    }
-                    f64_to(ds, sm[2 * k], sm[2 * k + 1]);
-                    f64_to(dq, sq[2 * k], sq[2 * k + 1]);
-                }
-                tmptx::tmem_st8(tcomp + 8 * h, sm);
-                tmptx::tmem_st8(tcomp + 32 + 8 * h, sq);
-            }
-            tmptx::tmem_wait_st();
-        } else if (two) {
-#pragma unroll
-            for (int r = 0; r < 16; r++) {
-                const float2 p = val(r);
-                fs[r] += p.x;
-                pq[r] = fmaf(p.x, p.x, pq[r]);
-                fs[r] += p.y;
-                pq[r] = fmaf(p.y, p.y, pq[r]);
-                bins(r);
-            }
-        } else {
-#pragma unroll
-            for (int r = 0; r < 16; r++) {
-                const float p = val(r).x;
-                fs[r] += p;
-                pq[r] = fmaf(p, p, pq[r]);
-                bins(r);
-            }
-        }
+        if (two) add(std::true_type{});
+        else add(std::false_type{});
         if (!PC::EXACT && (((i - i0) & 3) == 3 || i == npairs - 1)) {
             // Kahan: the compensation holds what the last addition added beyond its input
 #pragma unroll
